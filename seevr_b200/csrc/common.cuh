@@ -145,8 +145,6 @@ struct Scratch {
                             // (NULL: pairs taken in index order)
     uint32_t order_pairs;   // 1: pairs taken grouped by class (scene groups'
                             // handles), 0: in index order
-    uint32_t sweep_warps;   // warps per solver bundle: 2 in scene groups'
-                            // handles (64-wide passes), else 1
     uint32_t* lut_rep;      // [kLutHullMax] first body with a lookup per hull size
     uint32_t* lut_off;      // [max_bodies] lookup offset read by the narrowphase
     // solver, per contact
@@ -256,10 +254,9 @@ int launch_bundle_ranges(const World& w, const Scratch& s, cudaStream_t st);
 // Set the calling thread's message returned by seevr_last_error().
 void set_last_error(const char* msg);
 inline void set_last_error(const std::string& msg) { set_last_error(msg.c_str()); }
-// max_scene_bodies: the largest bundle; smem_bodies: bodies per bundle kept
-// in shared memory by the warp solver (larger bundles solve in place)
+// max_scene_bodies: the largest bundle
 int launch_solver(const World& w, const Consts& k, const Scratch& s, uint32_t mode,
-                  float dt, uint32_t max_scene_bodies, uint32_t smem_bodies, cudaStream_t st);
+                  float dt, uint32_t max_scene_bodies, cudaStream_t st);
 // Island-parallel solve of the whole contact list (needs s.isl); mode 0
 // sequential, 1 wavefront, 2 coloured.
 int launch_solver_islands(const World& w, const Consts& k, const Scratch& s, uint32_t mode,
@@ -270,7 +267,7 @@ int launch_solver_giant(const World& w, const Consts& k, const Scratch& s, float
                         cudaStream_t st);
 // Scenes above this many bodies are solved by islands (when allocated).
 constexpr uint32_t kWarpMaxBodies = 1024;
-constexpr uint32_t kRecWords = 10;  // float4 words of a warp-solver contact record
+constexpr uint32_t kRecWords = 10;  // float4 words of a bundle solver's contact record
 
 // One scene group's outputs, merged into the bound buffers at frame end
 // (physics.cu): its counters and status word, its pair and contact lists in

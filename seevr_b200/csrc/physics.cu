@@ -95,10 +95,6 @@ struct seevr_physics {
     uint32_t* body_bundle = nullptr;  // body -> bundle
     uint32_t num_bundles = 1;
     uint32_t max_bundle_bodies = 0;
-    // bodies per bundle the warp solver keeps in shared memory: the bundle
-    // size, so that single scenes above it (solved in place) do not cut
-    // the number of resident warps
-    uint32_t smem_bundle_bodies = 0;
     uint32_t num_scenes = 1;
     bool scenes_set = false;
     uint32_t single_scene_nb = 0xFFFFFFFFu;
@@ -397,7 +393,7 @@ struct FrameIssue {
         {
             const Range r("phys/pgs_solve");
             n += launch_solver(h->w, h->k, h->s, h->params.solver, sub_dt, h->max_bundle_bodies,
-                               h->smem_bundle_bodies, st);
+                               st);
         }
         T.end(kStSolve);
     }
@@ -677,7 +673,6 @@ seevr_status build_groups(seevr_physics* h) {
         g.h->s.wait_limit = h->s.wait_limit;
         g.h->s.giant_min = h->s.giant_min;
         g.h->s.order_pairs = 1;  // pairs by support path (narrowphase.cu)
-        g.h->s.sweep_warps = 2;  // 64-wide solver passes (solver.cu)
         st = seevr_physics_set_scenes(g.h, lo.data(), s1 - s0);
         if (st != SEEVR_OK) break;
         if (cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking) != cudaSuccess ||
@@ -790,7 +785,6 @@ seevr_status ensure_single_scene(seevr_physics* h, uint32_t nb, cudaStream_t st)
     h->single_scene_nb = nb;
     h->max_scene_bodies = nb;
     h->max_bundle_bodies = nb;
-    h->smem_bundle_bodies = nb;
     h->num_scenes = 1;
     h->num_bundles = 1;
     return SEEVR_OK;
@@ -1038,7 +1032,6 @@ seevr_status seevr_physics_set_scenes(seevr_physics* h, const uint32_t* body_off
     SEEVR_CUDA(cudaMemcpy(h->body_bundle, bs.data(), sizeof(uint32_t) * nb, cudaMemcpyHostToDevice));
     h->num_bundles = uint32_t(bundles.size() - 1);
     h->max_bundle_bodies = max_bundle;
-    h->smem_bundle_bodies = h->num_bundles > 1 ? std::min(max_bundle, target) : max_bundle;
     h->num_scenes = num_scenes;
     h->scenes_set = true;
     h->single_scene_nb = nb;

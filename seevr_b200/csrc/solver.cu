@@ -7,24 +7,24 @@
 // wavefront levels of different scenes simply merge); small scenes are
 // bundled so that a warp's lanes have work.
 //
-// One CTA per bundle.  Phase 1 stages the bundle's bodies (velocity, angular
-// velocity, rotation matrix, inverse inertia, inverse mass) in shared memory
-// (global scratch when the scene is too large).  Phase 2 computes, for every
-// contact in parallel, the values the reference recomputes on every
-// iteration but which cannot change during the solve: the lever arms
-// ra, rb (positions and contact points are constant), the normal effective
-// mass k, the friction coefficient and the restitution/Baumgarte bias
-// (taken from the pre-solve velocities, as physics.comp:504-521 does).
-// Phase 3 runs the Gauss-Seidel sweeps:
+// Per contact, the values the reference recomputes on every iteration but
+// which cannot change during the solve are computed once: the lever arms ra, rb
+// (positions and contact points are constant), the normal effective mass k, the
+// friction coefficient and the restitution/Baumgarte bias (taken from the
+// pre-solve velocities, as physics.comp:504-521 does).  Then the sweeps:
 //  - SEQUENTIAL: one thread, contacts in index order (physics.comp:523-582);
-//  - WAVEFRONT: contacts are assigned levels so that a contact comes after
-//    every earlier contact sharing a dynamic body with it; contacts of one
-//    level touch disjoint dynamic bodies and run in parallel.  Each contact
-//    then sees exactly the body state it sees in the sequential sweep, so the
-//    result is bit-identical to SEQUENTIAL.
+//  - WAVEFRONT: an update runs as soon as the earlier updates that share one of
+//    its dynamic bodies are done.  Each contact then sees exactly the body state
+//    it sees in the sequential sweep, so the result is bit-identical;
+//  - COLORED: the same with the contacts in the order of their greedy colours.
+// Bundles of up to kWarpMaxBodies bodies: k_solver_flow.  Larger scenes are solved
+// by islands (islands.cu), or without its work arrays by k_solver, one block over
+// levels of contacts.
 // A body is "fixed" when inv_mass == 0 and inv_inertia == 0: its velocities
 // cannot change (the reference writes v - 0*impulse, the same value), so
 // fixed bodies create no ordering constraint and are never written.
+#include <algorithm>
+
 #include "common.cuh"
 #include "solver.cuh"
 
@@ -198,404 +198,624 @@ __global__ void k_bundle_ranges(World w, uint32_t* __restrict__ bundle_c0) {
 }
 
 // ---- block per bundle -------------------------------------------------------
-// Bundles of up to kWarpMaxBodies bodies: one block of W warps per bundle;
-// one warp builds the levels and records, then the block sweeps passes of up
-// to 32 W same-level contacts, a barrier between passes.
-// What a solve round waits on lives in shared memory: the
-// bundle's velocities and angular velocities, the impulses and the level
-// boundaries.  The per-contact constants are computed directly in level
-// order, so the lanes of a round read consecutive entries.  Levels are
-// assigned 32 contacts at a time: each lane starts from the latest level of
-// its bodies in earlier chunks, then lanes are visited in order and every
-// later lane sharing a dynamic body with lane j moves past lane j's level.
-// One bundle per block: the SM places a bundle's 19 KB of shared memory
-// wherever it fits beside other kernels (14.05 -> 13.80 ms per frame
-// against four bundles per block on the 4,096-scene batch).
-// W = 1 for a handle stepped alone; W = 2 for scene groups' handles, whose
-// solver chains are the frame's critical path while other groups' collision
-// stages fill the GPU: 64-wide passes cut the largest bundles' passes per
-// iteration by about a tenth (frame 12.68 -> 12.13 ms with 8 groups on the
-// 4,096-scene batch), while alone the doubled warps per SM sub-partition
-// slow every pass more than that (12.52 -> 12.89 ms ungrouped).
-constexpr uint32_t kMaxSweepWarps = 2;
-constexpr uint32_t kWarpLamCap = 1024;   // impulses per bundle held in smem
-constexpr uint32_t kWarpLevelCap = 128;  // passes held in smem
-// pass entry: start position | count << kPassShift (count <= 128)
-constexpr uint32_t kPassShift = 24, kPassMask = (1u << kPassShift) - 1u;
-static_assert(32 * kMaxSweepWarps < (1u << (32 - kPassShift)), "pass count field too narrow");
-constexpr uint32_t kRegChunks = 8;  // contacts per lane kept in registers by the setup
+// Bundles of up to kWarpMaxBodies bodies: one block of W warps each, in dataflow
+// order.  In the sequential sweep the updates of one body's contacts follow each
+// other in contact order, iteration after iteration, and nothing else orders two
+// updates.  So every body counts the updates it has had, and the update of
+// contact c in iteration k may run as soon as each of its two dynamic bodies has
+// counted k d + r updates (d: the body's contacts, r: c's rank among them): it
+// then reads exactly the state it reads in the sequential sweep, and results are
+// bit for bit those of that sweep.  In every round the contacts that are ready
+// run together, whatever their iterations.  A sweep takes about (largest d)
+// rounds per iteration, where the levels of one iteration after another (7 to 11
+// for a settled 512-body pile, in 32-wide passes) took 8 to 22.  Contacts that
+// share no dynamic body with another (a third of a pile's) are taken apart: all
+// their iterations at once, beside the rounds.
+//
+// A bundle's time is the dependent chain of its rounds, and a round is bound by one
+// warp's latency and issue.  So a lane owns a contact for the whole solve, its
+// constants in registers; velocities and counts live in shared memory, both in
+// one 16-byte word per body; and the update's square root and divisions are
+// the branch-free ones of vmath.cuh: a warp where an argument is outside their
+// ranges redoes the update with the built-in ones.
+//
+// A lane owns contacts i, i + 32 W, ... and takes them in order, iteration after
+// iteration: the first unfinished update of the whole sequence is then at the
+// head of its lane's list and ready, so every round makes progress.
+constexpr uint32_t kInfoCap = 512;  // contacts whose bodies, ranks and positions fit in smem
+// a contact side's bundle-local body, flags and rank
+// (Free: the body is not written and orders nothing; Skip: both masses infinite)
+constexpr uint32_t kSideBody = 0xFFFu, kSideFree = 1u << 12, kSideSkip = 1u << 13, kRankShift = 16,
+                   kMaxRank = 0xFFFFu;
+static_assert(kWarpMaxBodies <= kSideBody, "body field too narrow");
 
-// A contact's record (kRecWords float4, 160 bytes): n ra rb bias kn mu,
-// both bodies' rotation matrix (columns), inverse inertia and inverse mass,
-// and the bundle-local body indices with each body's fixed flag in bit 31.
-// The matrices are those quat_to_mat gives at every update of the sweep,
-// built once here instead of at each of the 30 updates (a third fewer
-// instructions than rebuilding them from quaternions in the sweep).
-__device__ __forceinline__ void load_rec(const float4* __restrict__ src, float4 (&r)[kRecWords]) {
-#pragma unroll
-    for (uint32_t j = 0; j < kRecWords; ++j) r[j] = src[j];
+// What an update of a contact reads besides the velocities (physics.comp:504-521,
+// 533-546); kRecWords float4 in memory.
+struct Side {
+    f3 r, I;
+    m3 R;
+    float m;
+};
+struct Rec {
+    f3 n;
+    float bias, kn, rk, mu, msum;  // rk = 1 / kn, 0 when kn is out of div_by's range
+    Side a, b;
+};
+__device__ __forceinline__ Side load_side(const float4* p) {
+    const float4 c = p[0], d = p[1], e = p[2], f = p[3];
+    return Side{mk(c.x, c.y, c.z), mk(f.x, f.y, f.z),
+                m3{mk(c.w, d.x, d.y), mk(d.z, d.w, e.x), mk(e.y, e.z, e.w)}, f.w};
 }
-// Contact c's record at slot q (physics.comp:504-521, 533-546): the
-// constants, computed from the pre-solve velocities, and both bodies' data.
-__device__ __forceinline__ void write_rec(const World& w, const Consts& k, const Scratch& s,
-                                          const BodyView& B, uint32_t b0, uint32_t c, uint32_t la,
-                                          uint32_t lb, uint32_t q, float dt) {
+__device__ __forceinline__ void store_side(float4* p, const Side& s) {
+    p[0] = make_float4(s.r.x, s.r.y, s.r.z, s.R.c0.x);
+    p[1] = make_float4(s.R.c0.y, s.R.c0.z, s.R.c1.x, s.R.c1.y);
+    p[2] = make_float4(s.R.c1.z, s.R.c2.x, s.R.c2.y, s.R.c2.z);
+    p[3] = make_float4(s.I.x, s.I.y, s.I.z, s.m);
+}
+__device__ __forceinline__ Rec load_rec(const float4* p) {
+    const float4 a = p[0], b = p[1];
+    return Rec{mk(a.x, a.y, a.z), a.w, b.x, b.y, b.z, b.w, load_side(p + 2), load_side(p + 6)};
+}
+
+// Contact c's record: the constants, computed from the pre-solve velocities
+// (va, wa, vb, wb), and both bodies' data.  The rotation matrices are those
+// quat_to_mat gives at every update of the sweep, built once.
+__device__ __forceinline__ void make_rec(const World& w, const Consts& k, uint32_t c, uint32_t a,
+                                         uint32_t b, f3 va, f3 wa, f3 vb, f3 wb, float dt,
+                                         float4* out) {
     const uint32_t ga = w.c_a[c], gb = w.c_b[c];
-    const uint32_t a = b0 + la, b = b0 + lb;
     const f3 n = ld3(w.c_normal, c), cp = ld3(w.c_pos, c);
-    const f3 ra = sub(cp, ld3(w.pos, a)), rb = sub(cp, ld3(w.pos, b));
-    const f3 va = add(ld3(B.v, la), cross(ld3(B.w, la), ra));
-    const f3 vb = add(ld3(B.v, lb), cross(ld3(B.w, lb), rb));
-    const float vn = dot(sub(vb, va), n);
+    const Side A{sub(cp, ld3(w.pos, a)), ld3(w.inv_inertia, a), quat_to_mat(w.quat, a), w.inv_mass[a]};
+    const Side B{sub(cp, ld3(w.pos, b)), ld3(w.inv_inertia, b), quat_to_mat(w.quat, b), w.inv_mass[b]};
+    const f3 ua = add(va, cross(wa, A.r)), ub = add(vb, cross(wb, B.r));
+    const float vn = dot(sub(ub, ua), n);
     const float e = gmax(w.restitution[ga], w.restitution[gb]);
     const float bias = k.baumgarte * gmax(w.c_pen[c] - k.slop, 0.0f) / dt + e * gmax(-vn, 0.0f);
-    const float ima = B.invm[la], imb = B.invm[lb];
-    const float4 qa = make_float4(w.quat[size_t(a) * 4], w.quat[size_t(a) * 4 + 1],
-                                  w.quat[size_t(a) * 4 + 2], w.quat[size_t(a) * 4 + 3]);
-    const float4 qb = make_float4(w.quat[size_t(b) * 4], w.quat[size_t(b) * 4 + 1],
-                                  w.quat[size_t(b) * 4 + 2], w.quat[size_t(b) * 4 + 3]);
-    const m3 Ra = quat_to_mat(qa.x, qa.y, qa.z, qa.w), Rb = quat_to_mat(qb.x, qb.y, qb.z, qb.w);
-    const f3 Ia = ld3(B.invI, la), Ib = ld3(B.invI, lb);
-    const f3 ran = cross(ra, n), rbn = cross(rb, n);
-    const float kn = ima + imb + dot(ran, apply_inv_I(Ra, Ia, ran)) + dot(rbn, apply_inv_I(Rb, Ib, rbn));
-    float4* r = s.s_rec + size_t(q) * kRecWords;
-    r[0] = make_float4(n.x, n.y, n.z, ra.x);
-    r[1] = make_float4(ra.y, ra.z, rb.x, rb.y);
-    r[2] = make_float4(rb.z, bias, kn, sqrtf(w.friction[ga] * w.friction[gb]));
-    r[3] = make_float4(Ra.c0.x, Ra.c0.y, Ra.c0.z, Ra.c1.x);
-    r[4] = make_float4(Ra.c1.y, Ra.c1.z, Ra.c2.x, Ra.c2.y);
-    r[5] = make_float4(Ra.c2.z, Rb.c0.x, Rb.c0.y, Rb.c0.z);
-    r[6] = make_float4(Rb.c1.x, Rb.c1.y, Rb.c1.z, Rb.c2.x);
-    r[7] = make_float4(Rb.c2.y, Rb.c2.z, Ia.x, Ia.y);
-    r[8] = make_float4(Ia.z, Ib.x, Ib.y, Ib.z);
-    r[9] = make_float4(ima, imb, __uint_as_float(la | (is_fixed(B, la) ? 0x80000000u : 0u)),
-                       __uint_as_float(lb | (is_fixed(B, lb) ? 0x80000000u : 0u)));
+    const f3 ran = cross(A.r, n), rbn = cross(B.r, n);
+    const float msum = A.m + B.m;
+    const float kn = msum + dot(ran, apply_inv_I(A.R, A.I, ran)) + dot(rbn, apply_inv_I(B.R, B.I, rbn));
+    const float rk = kn >= kDivMin && kn <= kDivMax ? recip_of(kn, rcp_approx(kn)) : 0.0f;
+    out[0] = make_float4(n.x, n.y, n.z, bias);
+    out[1] = make_float4(kn, rk, sqrtf(w.friction[ga] * w.friction[gb]), msum);
+    store_side(out + 2, A);
+    store_side(out + 6, B);
 }
 
-// Passes of the positions [beg, pos) of one level, from entry npass on.
-// kPassWidth: contacts a pass solves at once (the block's threads).
-template <uint32_t kPassWidth>
-__device__ __forceinline__ uint32_t write_passes(uint32_t* gpass, uint32_t npass, uint32_t beg,
-                                                 uint32_t pos, uint32_t lane) {
-    for (uint32_t q = beg + lane * kPassWidth; q < pos; q += 32 * kPassWidth)
-        gpass[npass + (q - beg) / kPassWidth] = q | (min(kPassWidth, pos - q) << kPassShift);
-    return npass + (pos - beg + kPassWidth - 1) / kPassWidth;
-}
-
-__device__ __forceinline__ void solve_rec(float* V, float* W, const float4 (&r)[kRecWords], float* lam) {
-    const uint32_t xa = __float_as_uint(r[9].z), xb = __float_as_uint(r[9].w);
-    const m3 Ra{mk(r[3].x, r[3].y, r[3].z), mk(r[3].w, r[4].x, r[4].y), mk(r[4].z, r[4].w, r[5].x)};
-    const m3 Rb{mk(r[5].y, r[5].z, r[5].w), mk(r[6].x, r[6].y, r[6].z), mk(r[6].w, r[7].x, r[7].y)};
-    solve_core(V, W, xa & 0x7FFFFFFFu, xb & 0x7FFFFFFFu, (xa >> 31) != 0, (xb >> 31) != 0, r[9].x,
-               r[9].y, Ra, Rb, mk(r[7].z, r[7].w, r[8].x), mk(r[8].y, r[8].z, r[8].w),
-               mk(r[0].x, r[0].y, r[0].z), mk(r[0].w, r[1].x, r[1].y), mk(r[1].z, r[1].w, r[2].x),
-               r[2].y, r[2].z, r[2].w, lam);
-}
-
-__host__ __device__ constexpr uint32_t warp_smem_words(uint32_t nbmax) {
-    return 7 * nbmax + kWarpLamCap + kWarpLevelCap;
-}
-
-// Levels, solve positions, pass table and contact records of one bundle,
-// built by one warp (lane = its lane): returns the positions (contacts
-// solved) and the passes written to gpass.
-template <uint32_t kPassWidth>
-__device__ __forceinline__ void bundle_setup(const World& w, const Consts& k, const Scratch& s,
-                                             const BodyView& B, uint32_t mode, float dt,
-                                             uint32_t b0, uint32_t c0, uint32_t c1, uint32_t nbs,
-                                             uint32_t ncb, uint32_t* last, float* lam,
-                                             uint32_t* gpass, uint32_t lane, uint32_t& pos_out,
-                                             uint32_t& npass_out) {
-    const unsigned full = 0xFFFFFFFFu;
-    uint32_t maxl = 0, pos = 0, npass = 0;
-    if (mode != 2 && ncb <= 32 * kRegChunks && nbs <= 0x10000u) {
-        // ---- register path: each lane keeps its contacts (c0 + lane + 32 k)
-        // with their bodies (two 16-bit bundle-local indices, hence at most
-        // 65,536 bodies per bundle), levels and positions in registers
-        const uint32_t K = (ncb + 31) / 32;
-        uint32_t ab[kRegChunks], lv[kRegChunks], pk[kRegChunks];
-#pragma unroll
-        for (uint32_t j = 0; j < kRegChunks; ++j) {
-            const uint32_t c = c0 + 32 * j + lane;
-            ab[j] = 0xFFFFFFFFu;
-            if (j < K && c < c1)
-                ab[j] = (w.geom_body[w.c_a[c]] - b0) | ((w.geom_body[w.c_b[c]] - b0) << 16);
-        }
-#pragma unroll
-        for (uint32_t j = 0; j < kRegChunks; ++j) {
-            lv[j] = kNone;
-            if (j >= K) continue;  // warp-uniform
-            const bool valid = ab[j] != 0xFFFFFFFFu;
-            const uint32_t la = ab[j] & 0xFFFFu, lb = ab[j] >> 16;
-            // both inverse masses zero -> skipped (physics.comp:531)
-            const bool use = valid && !(B.invm[la] == 0.0f && B.invm[lb] == 0.0f);
-            uint32_t L = use ? 1u : 0u;
-            if (mode != 0) {
-                const bool da = use && !is_fixed(B, la), db = use && !is_fixed(B, lb);
-                const uint32_t xa = da ? la : (0x80000000u | (lane * 2u));
-                const uint32_t xb = db ? lb : (0x80000000u | (lane * 2u + 1u));
-                if (use) L = max(da ? last[la] : 0u, db ? last[lb] : 0u) + 1u;
-                for (uint32_t i = 0; i < 32; ++i) {
-                    const uint32_t ai = __shfl_sync(full, xa, i), bi = __shfl_sync(full, xb, i);
-                    const uint32_t Li = __shfl_sync(full, L, i);
-                    if (use && i < lane && (ai == xa || ai == xb || bi == xa || bi == xb))
-                        L = max(L, Li + 1u);
-                }
-                if (da) atomicMax(&last[la], L);
-                if (db) atomicMax(&last[lb], L);
-                __syncwarp();
-            }
-            if (use) lv[j] = L - 1u;
-            maxl = max(maxl, L);
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) maxl = max(maxl, __shfl_xor_sync(full, maxl, off));
-        const unsigned below = (1u << lane) - 1u;
-        for (uint32_t l = 0; l < maxl; ++l) {
-            const uint32_t beg = pos;
-#pragma unroll
-            for (uint32_t j = 0; j < kRegChunks; ++j) {
-                const bool hit = lv[j] == l;
-                const unsigned m = __ballot_sync(full, hit);
-                if (hit) pk[j] = pos + __popc(m & below);
-                pos += __popc(m);
-            }
-            npass = write_passes<kPassWidth>(gpass, npass, beg, pos, lane);
-        }
-#pragma unroll
-        for (uint32_t j = 0; j < kRegChunks; ++j) {
-            if (lv[j] == kNone) continue;
-            const uint32_t c = c0 + 32 * j + lane;
-            s.s_order[c0 + pk[j]] = c;
-            write_rec(w, k, s, B, b0, c, ab[j] & 0xFFFFu, ab[j] >> 16, c0 + pk[j], dt);
-            lam[pk[j]] = 0.0f;
-        }
+// One update (solve_core's operations in solve_core's order).  kBuiltin: with the
+// built-in square root and divisions; else the result tells whether every
+// argument was in the branch-free ones' ranges.
+template <bool kBuiltin>
+__device__ __forceinline__ bool update_core(const Rec& h, f3& va, f3& wa, f3& vb, f3& wb, float& lam) {
+    const Side &A = h.a, &B = h.b;
+    f3 ua = add(va, cross(wa, A.r)), ub = add(vb, cross(wb, B.r));
+    const float num = -dot(sub(ub, ua), h.n) + h.bias;
+    float d = kBuiltin ? num / h.kn : div_by(num, h.kn, h.rk);
+    const float ln = gmax(lam + d, 0.0f);
+    d = ln - lam;
+    lam = ln;
+    const f3 imp = scale(d, h.n);
+    va = sub(va, scale(A.m, imp));
+    vb = add(vb, scale(B.m, imp));
+    wa = sub(wa, apply_inv_I(A.R, A.I, cross(A.r, imp)));
+    wb = add(wb, apply_inv_I(B.R, B.I, cross(B.r, imp)));
+    // Coulomb friction along the current slip direction
+    ua = add(va, cross(wa, A.r));
+    ub = add(vb, cross(wb, B.r));
+    const f3 dv = sub(ub, ua);
+    const f3 vt = sub(dv, scale(dot(dv, h.n), h.n));
+    const float len2 = dot(vt, vt);
+    const float rs = rsqrt_approx(len2);
+    const float len = kBuiltin ? sqrtf(len2) : root_of(len2, rs);
+    // (1e-6)^2 lies in root_of's range; below it only the comparison matters
+    const bool still = len2 < kRootMin;
+    const bool slips = kBuiltin ? len > 1e-6f : !still && len > 1e-6f;
+    f3 td;
+    if (kBuiltin) {
+        td = divs(vt, len);
     } else {
-        // ---- memory path (colouring, or more contacts than the registers hold)
-        // ---- bodies of each contact; both inverse masses zero -> skipped (531)
-        for (uint32_t c = c0 + lane; c < c1; c += 32) {
-            const uint32_t la = w.geom_body[w.c_a[c]] - b0, lb = w.geom_body[w.c_b[c]] - b0;
-            const bool skip = B.invm[la] == 0.0f && B.invm[lb] == 0.0f;
-            s.s_ab[size_t(c) * 2] = skip ? kNone : la;
-            s.s_ab[size_t(c) * 2 + 1] = lb;
-        }
-        __syncwarp();
-
-        // ---- levels: colours (COLORED), wavefront levels (WAVEFRONT) or one
-        // level in index order (SEQUENTIAL)
-        bool coloured = mode == 2;
-        if (coloured) {
-            // greedy colouring in contact order: the smallest colour not used by
-            // an earlier contact at either of its dynamic bodies (per-body colour
-            // masks in `last`); more than 32 colours at a body falls back to the
-            // wavefront levels
-            uint32_t ok = 1u, mx = 0u;
-            if (lane == 0) {
-                for (uint32_t c = c0; c < c1; ++c) {
-                    const uint32_t la = s.s_ab[size_t(c) * 2], lb = s.s_ab[size_t(c) * 2 + 1];
-                    if (la == kNone) {
-                        s.s_level[c] = kNone;
-                        continue;
-                    }
-                    const bool da = !is_fixed(B, la), db = !is_fixed(B, lb);
-                    const uint32_t used = (da ? last[la] : 0u) | (db ? last[lb] : 0u);
-                    if (used == 0xFFFFFFFFu) {
-                        ok = 0u;
-                        break;
-                    }
-                    const uint32_t col = uint32_t(__ffs(int(~used))) - 1u;
-                    if (da) last[la] |= 1u << col;
-                    if (db) last[lb] |= 1u << col;
-                    s.s_level[c] = col;
-                    mx = max(mx, col + 1u);
-                }
-            }
-            ok = __shfl_sync(full, ok, 0);
-            maxl = __shfl_sync(full, mx, 0);
-            if (!ok) {
-                coloured = false;
-                maxl = 0;
-                for (uint32_t i = lane; i < nbs; i += 32) last[i] = 0;
-            }
-            __syncwarp();
-        }
-        for (uint32_t cb = c0; !coloured && cb < c1; cb += 32) {
-            const uint32_t c = cb + lane;
-            const bool valid = c < c1;
-            const uint32_t la = valid ? s.s_ab[size_t(c) * 2] : kNone;
-            const uint32_t lb = valid ? s.s_ab[size_t(c) * 2 + 1] : 0u;
-            const bool use = valid && la != kNone;
-            uint32_t L = use ? 1u : 0u;
-            if (mode != 0) {
-                const bool da = use && !is_fixed(B, la), db = use && !is_fixed(B, lb);
-                // dynamic bodies, or a sentinel unique to this lane and role
-                const uint32_t xa = da ? la : (0x80000000u | (lane * 2u));
-                const uint32_t xb = db ? lb : (0x80000000u | (lane * 2u + 1u));
-                if (use) L = max(da ? last[la] : 0u, db ? last[lb] : 0u) + 1u;
-                for (uint32_t j = 0; j < 32; ++j) {
-                    const uint32_t aj = __shfl_sync(full, xa, j), bj = __shfl_sync(full, xb, j);
-                    const uint32_t Lj = __shfl_sync(full, L, j);
-                    if (use && j < lane && (aj == xa || aj == xb || bj == xa || bj == xb))
-                        L = max(L, Lj + 1u);
-                }
-                if (da) atomicMax(&last[la], L);
-                if (db) atomicMax(&last[lb], L);
-            }
-            if (valid) s.s_level[c] = use ? L - 1u : kNone;
-            maxl = max(maxl, L);
-            __syncwarp();
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) maxl = max(maxl, __shfl_xor_sync(full, maxl, off));
-
-        // ---- positions: contacts grouped by level, index order within a level;
-        // passes: runs of at most kPassWidth positions of one level,
-        // the unit the lanes solve together.  A pass holds at least one contact,
-        // so the passes fit in [c0 + bundle, c1 + bundle] of s_lvl_start.
-        for (uint32_t l = 0; l < maxl; ++l) {
-            const uint32_t beg = pos;
-            for (uint32_t cb = c0; cb < c1; cb += 32) {
-                const uint32_t c = cb + lane;
-                const bool hit = c < c1 && s.s_level[c] == l;
-                const unsigned m = __ballot_sync(full, hit);
-                if (hit) s.s_order[c0 + pos + __popc(m & ((1u << lane) - 1u))] = c;
-                pos += __popc(m);
-            }
-            npass = write_passes<kPassWidth>(gpass, npass, beg, pos, lane);
-        }
-        __syncwarp();
-        for (uint32_t i = lane; i < pos; i += 32) {
-            const uint32_t c = s.s_order[c0 + i];
-            write_rec(w, k, s, B, b0, c, s.s_ab[size_t(c) * 2], s.s_ab[size_t(c) * 2 + 1], c0 + i, dt);
-            lam[i] = 0.0f;
-        }
+        const float rl = recip_of(len, recip_of(len, rs));  // rs: two ulps off at worst
+        td = mk(div_by(vt.x, len, rl), div_by(vt.y, len, rl), div_by(vt.z, len, rl));
     }
-    pos_out = pos;
-    npass_out = npass;
+    const f3 rat = cross(A.r, td), rbt = cross(B.r, td);
+    const float kt = h.msum + dot(rat, apply_inv_I(A.R, A.I, rat)) + dot(rbt, apply_inv_I(B.R, B.I, rbt));
+    const float dl = gmin(kBuiltin ? len / kt : div_by(len, kt, recip_of(kt, rcp_approx(kt))),
+                          h.mu * ln);
+    const f3 it = scale(dl, td);
+    const f3 va2 = add(va, scale(A.m, it)), vb2 = sub(vb, scale(B.m, it));
+    const f3 wa2 = add(wa, apply_inv_I(A.R, A.I, cross(A.r, it)));
+    const f3 wb2 = sub(wb, apply_inv_I(B.R, B.I, cross(B.r, it)));
+    if (slips) {
+        va = va2;
+        vb = vb2;
+        wa = wa2;
+        wb = wb2;
+    }
+    if (kBuiltin) return true;
+    // a NaN fails every comparison; the slip's components are at most len
+    const uint32_t key = min(min(size_key(vt.x), size_key(vt.y)), size_key(vt.z));
+    return h.rk != 0.0f && size_key(num) >= kNumMinKey && fabsf(num) <= kNumMax &&
+           (still || (len2 <= kRootMax && key >= kNumMinKey && kt >= kDivMin && kt <= kDivMax));
 }
 
-// Barrier of a W-warp block.
+// A contact's velocities and impulse during the solve.
+struct State {
+    f3 va, wa, vb, wb;
+    float lam;
+};
+__device__ __noinline__ void update_builtin(const Rec* h, State* x) {
+    update_core<true>(*h, x->va, x->wa, x->vb, x->wb, x->lam);
+}
+// The update of the lanes that count (the others' result is not used).
+__device__ __forceinline__ State update(const Rec& h, bool counts, const State& x) {
+    State y = x;
+    const bool ok = update_core<false>(h, y.va, y.wa, y.vb, y.wb, y.lam);
+    if (counts && !ok) {
+        const Rec copy = h;
+        State z = x;
+        update_builtin(&copy, &z);
+        y = z;
+    }
+    return y;
+}
+
+// Shared memory of a block: per body its velocity with the count of its updates
+// and its angular velocity (a float4 each), the contact sides' words, and records
+// of `recs` contacts for pairs that own several.
+__host__ __device__ constexpr uint32_t flow_smem_bytes(uint32_t nbmax, uint32_t recs) {
+    return 32 * nbmax + 12 * kInfoCap + 16 * kRecWords * recs;
+}
+struct FlowBodies {
+    float4* v;  // velocity, updates counted (bits of an integer)
+    float4* w;  // angular velocity, unused
+    __device__ __forceinline__ uint32_t* count(uint32_t l) const {
+        return reinterpret_cast<uint32_t*>(&v[l].w);
+    }
+};
+
+__device__ __forceinline__ float4 ld4(const float4* p) {  // shared memory
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(uint32_t(__cvta_generic_to_shared(p)))
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ void st4(float4* p, float4 v) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(
+                     uint32_t(__cvta_generic_to_shared(p))),
+                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+
+// Barrier of the block's first `threads` threads.
 template <uint32_t W>
-__device__ __forceinline__ void block_sync() {
-    if (W == 1)
+__device__ __forceinline__ void part_sync(uint32_t threads) {
+    if (W == 1 || threads == 32)
         __syncwarp();
     else
-        __syncthreads();
+        __barrier_sync_count(1, threads);
 }
 
+// Ranks of the contact sides in info[0 .. 2 nc), contact order, by one warp:
+// 16 contacts at a time.  The bodies' counts (zero before) end as their
+// contacts.  False when a rank does not fit its field.
+__device__ __forceinline__ bool rank_sides(uint32_t* info, const FlowBodies& B, uint32_t nc) {
+    const uint32_t lane = threadIdx.x & 31u;
+    bool fits = true;
+    for (uint32_t e0 = 0; e0 < 2 * nc; e0 += 32) {
+        const uint32_t e = e0 + lane;
+        const uint32_t x = e < 2 * nc ? info[e] : kSideFree;
+        const bool counts = !(x & kSideFree);
+        const uint32_t body = x & kSideBody;
+        const unsigned m = __match_any_sync(0xFFFFFFFFu, counts ? body : 0x80000000u | lane);
+        if (counts) {
+            const uint32_t r = *B.count(body) + __popc(m & ((1u << lane) - 1u));
+            fits &= r < kMaxRank;
+            info[e] = (x & 0xFFFFu) | (r << kRankShift);
+        }
+        __syncwarp();
+        if (counts && lane == uint32_t(__ffs(m)) - 1u) *B.count(body) += __popc(m);
+        __syncwarp();
+    }
+    return __all_sync(0xFFFFFFFFu, fits);
+}
+
+// COLORED order: greedy colours in contact order (the smallest colour not used
+// by an earlier contact at either dynamic body; masks in the bodies' counts),
+// contacts sorted by colour in order[0 .. nc), ranks by colour.  False when a
+// body needs more than 32 colours.  One warp; level: scratch.
+__device__ __forceinline__ bool colour_sides(uint32_t* info, const FlowBodies& B, uint32_t nc,
+                                             uint32_t* level, uint32_t* order) {
+    const unsigned full = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t ok = 1u, mx = 0u;
+    if (lane == 0)
+        for (uint32_t i = 0; i < nc && ok; ++i) {
+            const uint32_t a = info[2 * i], b = info[2 * i + 1];
+            if (a & kSideSkip) {
+                level[i] = 0u;  // solved by nobody: any colour
+                continue;
+            }
+            const uint32_t used = (a & kSideFree ? 0u : *B.count(a & kSideBody)) |
+                                  (b & kSideFree ? 0u : *B.count(b & kSideBody));
+            ok = used != 0xFFFFFFFFu;
+            const uint32_t col = uint32_t(__ffs(int(~used))) - 1u;
+            if (ok && !(a & kSideFree)) *B.count(a & kSideBody) |= 1u << col;
+            if (ok && !(b & kSideFree)) *B.count(b & kSideBody) |= 1u << col;
+            level[i] = col;
+            mx = max(mx, col + 1u);
+        }
+    ok = __shfl_sync(full, ok, 0);
+    mx = __shfl_sync(full, mx, 0);
+    __syncwarp();
+    if (!ok) return false;
+    for (uint32_t e = lane; e < 2 * nc; e += 32) {
+        const uint32_t x = info[e];
+        if (!(x & kSideFree))
+            info[e] = (x & 0xFFFFu) |
+                      (__popc(*B.count(x & kSideBody) & ((1u << level[e >> 1]) - 1u)) << kRankShift);
+    }
+    uint32_t pos = 0;
+    for (uint32_t l = 0; l < max(mx, 1u); ++l)
+        for (uint32_t i0 = 0; i0 < nc; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            const bool hit = i < nc && level[i] == l;
+            const unsigned m = __ballot_sync(full, hit);
+            if (hit) order[pos + __popc(m & ((1u << lane) - 1u))] = i;
+            pos += __popc(m);
+        }
+    __syncwarp();
+    return true;
+}
+
+// Positions: first the contacts that share a dynamic body with another one
+// (their count is returned), then the lone ones.  With a lane for each (at most
+// `lanes`), the former go by falling degree (the larger of the two bodies'), so
+// that the longest chains share few warps; lanes that own several need the
+// sequence's order, which `seq` gives (NULL: contact order).  One warp.
+__device__ __forceinline__ uint32_t order_contacts(const uint32_t* info, const FlowBodies& B,
+                                                   uint32_t nc, uint32_t lanes, const uint32_t* seq,
+                                                   uint32_t* order) {
+    const unsigned full = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u;
+    auto degree = [&](uint32_t i) {
+        const uint32_t a = info[2 * i], b = info[2 * i + 1];
+        return max(a & kSideFree ? 0u : *B.count(a & kSideBody),
+                   b & kSideFree ? 0u : *B.count(b & kSideBody));
+    };
+    uint32_t chained = 0;
+    for (uint32_t i0 = 0; i0 < nc; i0 += 32)
+        chained += __popc(__ballot_sync(full, i0 + lane < nc && degree(min(i0 + lane, nc - 1)) > 1u));
+    // classes: degrees 4 and above, 3, 2, lone ones; or all chained ones, lone ones
+    // one warp alone runs the lone ones in the same rounds
+    if (lanes == 32u && nc <= lanes) {
+        if (lane < nc) order[lane] = lane;
+        return nc;
+    }
+    const bool one_each = chained <= lanes;
+    uint32_t pos = 0;
+    for (uint32_t cls = 4; cls > 0; --cls) {
+        if (!one_each && (cls == 3u || cls == 2u)) continue;
+        for (uint32_t i0 = 0; i0 < nc; i0 += 32) {
+            const bool valid = i0 + lane < nc;
+            const uint32_t i = valid ? (!one_each && seq ? seq[i0 + lane] : i0 + lane) : 0u;
+            const uint32_t d = degree(i);
+            const bool hit = valid && (cls == 1u   ? d <= 1u
+                                       : !one_each ? d > 1u
+                                       : cls == 4u ? d >= 4u
+                                                   : d == cls);
+            const unsigned m = __ballot_sync(full, hit);
+            if (hit) order[pos + __popc(m & ((1u << lane) - 1u))] = i;
+            pos += __popc(m);
+        }
+    }
+    return chained;
+}
+
+struct FlowArgs {
+    uint32_t c0, nc, slot, width, threads, iters;  // nc: chained contacts
+    const uint32_t* order;  // contact (from c0) of each position
+    const uint32_t* info;
+    const float4* rec;  // records by contact
+    uint32_t* left;     // lanes that are not done
+};
+
+// The rounds of one bundle's chained contacts.  kSeveral: lanes own more than one.
+template <uint32_t W, bool kSeveral>
+__device__ __forceinline__ void flow_sweep(const World& w, const Scratch& s, const FlowArgs& f,
+                                           const FlowBodies& B) {
+    const unsigned full = 0xFFFFFFFFu;
+    uint32_t i = f.slot, it = 0, c = f.order[min(i, f.nc - 1)];
+    Rec h = load_rec(f.rec + size_t(c) * kRecWords);
+    uint32_t xa = f.info[2 * c], xb = f.info[2 * c + 1];
+    uint32_t da = 0, db = 0, ka = 0, kb = 0;  // degrees, counts to wait for
+    State x{};
+    bool live = i < f.nc && f.iters > 0 && !(xa & kSideSkip);
+    auto degree = [&](uint32_t y) { return y & kSideFree ? 0u : *B.count(y & kSideBody); };
+    // counts start at the body's contacts (the ranking's result)
+    auto arm = [&] {
+        if (kSeveral) {
+            const size_t at = size_t(f.c0 + c) * 2;
+            da = s.s_abp[at];
+            db = s.s_abp[at + 1];
+        }
+        ka = da * (it + 1) + (xa >> kRankShift);
+        kb = db * (it + 1) + (xb >> kRankShift);
+        const float4 va = ld4(B.v + (xa & kSideBody)), wa = ld4(B.w + (xa & kSideBody)),
+                     vb = ld4(B.v + (xb & kSideBody)), wb = ld4(B.w + (xb & kSideBody));
+        x.va = mk(va.x, va.y, va.z);
+        x.wa = mk(wa.x, wa.y, wa.z);
+        x.vb = mk(vb.x, vb.y, vb.z);
+        x.wb = mk(wb.x, wb.y, wb.z);
+    };
+    if (kSeveral) {
+        // the degrees of the lane's contacts, before the counts move on
+        for (uint32_t j = i; j < f.nc; j += f.width) {
+            const uint32_t e = f.order[j];
+            s.s_abp[size_t(f.c0 + e) * 2] = degree(f.info[2 * e]);
+            s.s_abp[size_t(f.c0 + e) * 2 + 1] = degree(f.info[2 * e + 1]);
+        }
+    } else {
+        da = degree(xa);
+        db = degree(xb);
+    }
+    if (live) {
+        arm();
+        atomicAdd(f.left, 1u);
+    }
+    part_sync<W>(f.threads);
+    // the first unfinished update of the sequence is ready in every round, so
+    // iters * nc rounds are enough
+    for (uint64_t round = 0, cap = uint64_t(f.iters) * f.nc; round <= cap; ++round) {
+        // a body that no other contact moves keeps its velocities in registers
+        bool ready = live;
+        const uint32_t la = xa & kSideBody, lb = xb & kSideBody;
+        if (live && (kSeveral || da > 1u) && !(xa & kSideFree)) {
+            const float4 v = ld4(B.v + la), o = ld4(B.w + la);
+            ready = __float_as_uint(v.w) == ka;
+            x.va = mk(v.x, v.y, v.z);
+            x.wa = mk(o.x, o.y, o.z);
+        }
+        if (live && (kSeveral || db > 1u) && !(xb & kSideFree)) {
+            const float4 v = ld4(B.v + lb), o = ld4(B.w + lb);
+            ready = ready && __float_as_uint(v.w) == kb;
+            x.vb = mk(v.x, v.y, v.z);
+            x.wb = mk(o.x, o.y, o.z);
+        }
+        const uint32_t left = *f.left;
+        part_sync<W>(f.threads);  // every read of the round before its writes
+        if (left == 0u) break;
+        if (__any_sync(full, ready)) {
+            const State y = update(h, ready, x);
+            if (ready) {
+                x.lam = y.lam;
+                if (!(xa & kSideFree)) {
+                    x.va = y.va;
+                    x.wa = y.wa;
+                    st4(B.w + la, make_float4(y.wa.x, y.wa.y, y.wa.z, 0.0f));
+                    st4(B.v + la, make_float4(y.va.x, y.va.y, y.va.z, __uint_as_float(ka + 1u)));
+                }
+                if (!(xb & kSideFree)) {
+                    x.vb = y.vb;
+                    x.wb = y.wb;
+                    st4(B.w + lb, make_float4(y.wb.x, y.wb.y, y.wb.z, 0.0f));
+                    st4(B.v + lb, make_float4(y.vb.x, y.vb.y, y.vb.z, __uint_as_float(kb + 1u)));
+                }
+                if (kSeveral) {  // on to the lane's next contact
+                    w.lambda[f.c0 + c] = x.lam;
+                    i += f.width;
+                    if (i >= f.nc) {
+                        i = f.slot;
+                        live = ++it < f.iters;
+                    }
+                    if (live) {
+                        c = f.order[i];
+                        h = load_rec(f.rec + size_t(c) * kRecWords);
+                        xa = f.info[2 * c];
+                        xb = f.info[2 * c + 1];
+                        x.lam = w.lambda[f.c0 + c];
+                        arm();
+                    }
+                } else {
+                    live = ++it < f.iters;
+                    ka += da;
+                    kb += db;
+                }
+            }
+            const unsigned done = __ballot_sync(full, ready && !live);
+            if (done && (threadIdx.x & 31u) == 0u) atomicSub(f.left, uint32_t(__popc(done)));
+        }
+        part_sync<W>(f.threads);
+    }
+    if (!kSeveral && i < f.nc) w.lambda[f.c0 + c] = x.lam;
+}
+
+// The lone contacts (no other contact at their dynamic bodies): all their
+// iterations at once, 32 contacts per warp, the batches by ticket.
+__device__ __forceinline__ void lone_sweep(const World& w, const FlowArgs& f, const FlowBodies& B,
+                                           uint32_t total, uint32_t* ticket) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (;;) {
+        uint32_t b = 0;
+        if (lane == 0) b = atomicAdd(ticket, 1u);
+        b = f.nc + 32 * __shfl_sync(0xFFFFFFFFu, b, 0);
+        if (b >= total) return;
+        if (b + lane >= total) continue;
+        const uint32_t c = f.order[b + lane], xa = f.info[2 * c], xb = f.info[2 * c + 1];
+        if (xa & kSideSkip) continue;
+        const Rec h = load_rec(f.rec + size_t(c) * kRecWords);
+        const uint32_t la = xa & kSideBody, lb = xb & kSideBody;
+        const float4 va = ld4(B.v + la), wa = ld4(B.w + la), vb = ld4(B.v + lb), wb = ld4(B.w + lb);
+        State x{mk(va.x, va.y, va.z), mk(wa.x, wa.y, wa.z), mk(vb.x, vb.y, vb.z),
+                mk(wb.x, wb.y, wb.z), 0.0f};
+        for (uint32_t it = 0; it < f.iters; ++it) {
+            const State y = update(h, true, x);
+            x.lam = y.lam;
+            if (!(xa & kSideFree)) {  // a fixed body keeps its velocities
+                x.va = y.va;
+                x.wa = y.wa;
+            }
+            if (!(xb & kSideFree)) {
+                x.vb = y.vb;
+                x.wb = y.wb;
+            }
+        }
+        if (!(xa & kSideFree)) {
+            st4(B.v + la, make_float4(x.va.x, x.va.y, x.va.z, 0.0f));
+            st4(B.w + la, make_float4(x.wa.x, x.wa.y, x.wa.z, 0.0f));
+        }
+        if (!(xb & kSideFree)) {
+            st4(B.v + lb, make_float4(x.vb.x, x.vb.y, x.vb.z, 0.0f));
+            st4(B.w + lb, make_float4(x.wb.x, x.wb.y, x.wb.z, 0.0f));
+        }
+        w.lambda[f.c0 + c] = x.lam;
+    }
+}
+
+// nbmax: bodies of the largest bundle; recs: contact records that fit in shared
+// memory.
 template <uint32_t W>
-__global__ void __launch_bounds__(32 * W)
-    k_solver_warp(World w, Consts k, Scratch s, uint32_t mode, float dt, uint32_t nbmax) {
-    constexpr uint32_t kSweepThreads = 32 * W;
-    // nbmax: bodies per warp held in shared memory; a bundle with more
-    // bodies (a single scene above the bundle size) solves on the bound
-    // velocity buffers in place
-    extern __shared__ float sm[];
+__global__ void __launch_bounds__(32 * W, 12 / W)
+    k_solver_flow(World w, Consts k, Scratch s, uint32_t mode, float dt, uint32_t nbmax,
+                  uint32_t recs) {
+    constexpr uint32_t kThreads = 32 * W;
+    extern __shared__ float4 sm4[];
+    __shared__ uint32_t sh_order, sh_left, sh_chained, sh_ticket;
     if (halted(w.status)) return;  // contacts from a scan that gave up
     const uint32_t t = threadIdx.x, lane = t & 31u, wid = t >> 5;
     const uint32_t bundle = blockIdx.x;
     if (bundle >= w.nbundles) return;
-    const uint32_t b0 = w.bundle_off[bundle], b1 = w.bundle_off[bundle + 1];
     const uint32_t c0 = s.bundle_c0[bundle], c1 = s.bundle_c0[bundle + 1];
+    const uint32_t b0 = w.bundle_off[bundle], b1 = w.bundle_off[bundle + 1];
     if (c0 >= c1) return;
-    const uint32_t nbs = b1 - b0, ncb = c1 - c0;
-    // pass entries hold a position in kPassShift bits: a bundle with more
-    // contacts runs the sequential sweep, which has no pass table and gives
-    // the same result bit for bit
-    if (ncb > kPassMask) mode = 0;
+    const uint32_t nbs = b1 - b0, nc = c1 - c0;
+    const FlowBodies B{sm4, sm4 + nbmax};
+    uint32_t* info = nc <= kInfoCap ? reinterpret_cast<uint32_t*>(sm4 + 2 * nbmax)
+                                    : s.s_ab + size_t(c0) * 2;
+    // (s_level: the colours of mode 2 are done with when the positions are made)
+    uint32_t* order = nc <= kInfoCap ? reinterpret_cast<uint32_t*>(sm4 + 2 * nbmax + kInfoCap / 2)
+                                     : s.s_level + c0;
+    float4* rec = nc <= recs ? sm4 + 2 * nbmax + kInfoCap / 2 + kInfoCap / 4
+                             : s.s_rec + size_t(c0) * kRecWords;
 
-    float* base = sm;
-    const bool in_smem = nbs <= nbmax;
-    float* V = in_smem ? base : w.vel + size_t(b0) * 3;
-    float* Wv = in_smem ? base + 3 * nbmax : w.omega + size_t(b0) * 3;
-    uint32_t* last = in_smem ? reinterpret_cast<uint32_t*>(base + 6 * nbmax) : s.s_last + b0;
-    float* lam = ncb <= kWarpLamCap ? base + 7 * nbmax : s.s_lam + c0;
-    uint32_t* lvl_sm = reinterpret_cast<uint32_t*>(base + 7 * nbmax + kWarpLamCap);
-    for (uint32_t i = t; i < nbs; i += kSweepThreads) {
-        if (in_smem) {
-            st3(V, i, ld3(w.vel, b0 + i));
-            st3(Wv, i, ld3(w.omega, b0 + i));
+    // ---- the bundle's bodies; every contact side's body and flags ----
+    for (uint32_t i = t; i < nc; i += kThreads) {
+        const uint32_t a = w.geom_body[w.c_a[c0 + i]], b = w.geom_body[w.c_b[c0 + i]];
+        const float ma = w.inv_mass[a], mb = w.inv_mass[b];
+        const f3 Ia = ld3(w.inv_inertia, a), Ib = ld3(w.inv_inertia, b);
+        const bool fa = ma == 0.0f && Ia.x == 0.0f && Ia.y == 0.0f && Ia.z == 0.0f;
+        const bool fb = mb == 0.0f && Ib.x == 0.0f && Ib.y == 0.0f && Ib.z == 0.0f;
+        uint32_t xa = a - b0, xb = b - b0;
+        if (ma == 0.0f && mb == 0.0f) {  // skipped (physics.comp:531)
+            xa |= kSideSkip | kSideFree;
+            xb |= kSideSkip | kSideFree;
+        } else {
+            if (fa || a == b) xa |= kSideFree;  // both sides one body: b is written last
+            if (fb) xb |= kSideFree;
         }
-        last[i] = 0;
+        info[2 * i] = xa;
+        info[2 * i + 1] = xb;
     }
-    block_sync<W>();
-    BodyView B{V, Wv, nullptr, w.inv_inertia + size_t(b0) * 3, w.inv_mass + b0};
+    for (uint32_t i = t; i < nbs; i += kThreads) {
+        const f3 v = ld3(w.vel, b0 + i), om = ld3(w.omega, b0 + i);
+        B.v[i] = make_float4(v.x, v.y, v.z, 0.0f);
+        B.w[i] = make_float4(om.x, om.y, om.z, 0.0f);
+    }
+    if (t == 0) sh_left = sh_ticket = 0;
+    __syncthreads();
 
-    uint32_t* gpass = s.s_lvl_start + c0 + bundle;
-    uint32_t pos = 0, npass = 0;
-    if (W == 1) {
-        bundle_setup<kSweepThreads>(w, k, s, B, mode, dt, b0, c0, c1, nbs, ncb, last, lam, gpass,
-                                    lane, pos, npass);
-        __syncwarp();
-    } else {
-        __shared__ uint32_t sh_counts[2];
-        if (wid == 0) {
-            bundle_setup<kSweepThreads>(w, k, s, B, mode, dt, b0, c0, c1, nbs, ncb, last, lam,
-                                        gpass, lane, pos, npass);
-            if (lane == 0) {
-                sh_counts[0] = pos;
-                sh_counts[1] = npass;
-            }
+    // ---- ranks and positions by the last warp, records by the others ----
+    if (wid == W - 1) {
+        bool coloured = mode == 2, ok = true;
+        if (coloured && !colour_sides(info, B, nc, s.s_level + c0, s.s_order + c0)) {
+            coloured = false;  // contact order instead
+            for (uint32_t i = lane; i < nbs; i += 32) *B.count(i) = 0;
+            __syncwarp();
         }
-        __syncthreads();
-        pos = sh_counts[0];
-        npass = sh_counts[1];
+        if (mode != 0 && !coloured) ok = rank_sides(info, B, nc);
+        if (coloured) {
+            __syncwarp();
+            for (uint32_t i = lane; i < nbs; i += 32) *B.count(i) = __popc(*B.count(i));
+            __syncwarp();
+        }
+        uint32_t chained = 0;
+        if (mode != 0) {
+            __syncwarp();
+            chained = order_contacts(info, B, nc, kThreads, coloured ? s.s_order + c0 : nullptr, order);
+        }
+        // contacts one by one, the reference's loop, when the ranks are too large
+        if (lane == 0) {
+            sh_order = mode != 0 && ok;
+            sh_chained = chained;
+        }
     }
-    const bool pass_sm = npass <= kWarpLevelCap;
-    if (pass_sm)
-        for (uint32_t j = t; j < npass; j += kSweepThreads) lvl_sm[j] = gpass[j];
-    block_sync<W>();
-    const uint32_t* pass = pass_sm ? lvl_sm : gpass;
+    if (W == 1 || wid < W - 1)
+        for (uint32_t i = t; i < nc; i += 32 * (W == 1 ? 1 : W - 1)) {
+            const uint32_t la = info[2 * i] & kSideBody, lb = info[2 * i + 1] & kSideBody;
+            const float4 va = B.v[la], wa = B.w[la], vb = B.v[lb], wb = B.w[lb];
+            make_rec(w, k, c0 + i, b0 + la, b0 + lb, mk(va.x, va.y, va.z), mk(wa.x, wa.y, wa.z),
+                     mk(vb.x, vb.y, vb.z), mk(wb.x, wb.y, wb.z), dt, rec + size_t(i) * kRecWords);
+        }
+    __syncthreads();
 
-    // ---- Gauss-Seidel sweeps ----
-    if (mode == 0) {
-        if (t == 0) {
-            float4 r[kRecWords];
+    if (!sh_order) {
+        // ---- SEQUENTIAL: the reference order, one lane ----
+        if (t == 0)
             for (uint32_t it = 0; it < k.pgs_iterations; ++it)
-                for (uint32_t i = 0; i < pos; ++i) {
-                    load_rec(s.s_rec + size_t(c0 + i) * kRecWords, r);
-                    solve_rec(V, Wv, r, &lam[i]);
+                for (uint32_t i = 0; i < nc; ++i) {
+                    const uint32_t xa = info[2 * i], xb = info[2 * i + 1];
+                    if (xa & kSideSkip) continue;
+                    const uint32_t la = xa & kSideBody, lb = xb & kSideBody;
+                    const float4 va = B.v[la], wa = B.w[la], vb = B.v[lb], wb = B.w[lb];
+                    const State x = update(load_rec(rec + size_t(i) * kRecWords), true,
+                                           State{mk(va.x, va.y, va.z), mk(wa.x, wa.y, wa.z),
+                                                 mk(vb.x, vb.y, vb.z), mk(wb.x, wb.y, wb.z),
+                                                 w.lambda[c0 + i]});
+                    if (!(xa & kSideFree)) {
+                        B.v[la] = make_float4(x.va.x, x.va.y, x.va.z, 0.0f);
+                        B.w[la] = make_float4(x.wa.x, x.wa.y, x.wa.z, 0.0f);
+                    }
+                    if (!(xb & kSideFree)) {
+                        B.v[lb] = make_float4(x.vb.x, x.vb.y, x.vb.z, 0.0f);
+                        B.w[lb] = make_float4(x.wb.x, x.wb.y, x.wb.z, 0.0f);
+                    }
+                    w.lambda[c0 + i] = x.lam;
                 }
+    } else {
+        // contacts go to the warps from a different one on in each block, so that
+        // the longest chains of an SM's blocks do not meet on one scheduler
+        const uint32_t role = (wid + bundle) % W, chained = sh_chained;
+        const FlowArgs f{c0,   chained, role * 32 + lane, kThreads, 32u * min(W, (chained + 31) / 32),
+                         k.pgs_iterations, order, info, rec, &sh_left};
+        if (role * 32 < chained) {  // dataflow rounds, by the warps that own chained contacts
+            if (chained > kThreads)
+                flow_sweep<W, true>(w, s, f, B);
+            else
+                flow_sweep<W, false>(w, s, f, B);
         }
-    } else if (npass > 0) {
-        // the next pass's records are loaded while this pass solves
-        float4 cur[kRecWords], nxt[kRecWords];
-        uint32_t pe = pass[0];
-        if (t < (pe >> kPassShift))
-            load_rec(s.s_rec + size_t(c0 + (pe & kPassMask) + t) * kRecWords, nxt);
-        const uint32_t total = k.pgs_iterations * npass;
-        uint32_t p = 0;
-        for (uint32_t q = 0; q < total; ++q) {
-#pragma unroll
-            for (uint32_t j = 0; j < kRecWords; ++j) cur[j] = nxt[j];
-            const uint32_t ce = pe;
-            p = p + 1 == npass ? 0u : p + 1;
-            pe = pass[p];
-            if (q + 1 < total && t < (pe >> kPassShift))
-                load_rec(s.s_rec + size_t(c0 + (pe & kPassMask) + t) * kRecWords, nxt);
-            if (t < (ce >> kPassShift)) solve_rec(V, Wv, cur, &lam[(ce & kPassMask) + t]);
-            block_sync<W>();
-        }
+        lone_sweep(w, f, B, nc, &sh_ticket);
     }
-    block_sync<W>();
-    // ---- results back to the bound buffers ----
-    if (in_smem)
-        for (uint32_t i = t; i < nbs; i += kSweepThreads) {
-            st3(w.vel, b0 + i, ld3(V, i));
-            st3(w.omega, b0 + i, ld3(Wv, i));
-        }
-    for (uint32_t i = t; i < pos; i += kSweepThreads) w.lambda[s.s_order[c0 + i]] = lam[i];
+    __syncthreads();
+    // ---- velocities back to the bound buffers ----
+    for (uint32_t i = t; i < nbs; i += kThreads) {
+        const float4 v = B.v[i], om = B.w[i];
+        st3(w.vel, b0 + i, mk(v.x, v.y, v.z));
+        st3(w.omega, b0 + i, mk(om.x, om.y, om.z));
+    }
 }
 
 constexpr uint32_t kSolverMaxSmem = 160 * 1024;
+constexpr uint32_t kFlowMaxSmem = 120 * 1024;
 
 cudaError_t init_solver() {
-    const int bytes = int(warp_smem_words(kWarpMaxBodies) * sizeof(float));
-    cudaError_t e = cudaFuncSetAttribute(k_solver_warp<1>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_solver_warp<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
+    for (const void* f : {reinterpret_cast<const void*>(k_solver_flow<1>),
+                          reinterpret_cast<const void*>(k_solver_flow<2>),
+                          reinterpret_cast<const void*>(k_solver_flow<4>),
+                          reinterpret_cast<const void*>(k_solver_flow<8>)}) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFlowMaxSmem));
+        if (e != cudaSuccess) return e;
+    }
     // opt in to more than 48 KB of dynamic shared memory; done at handle
     // creation so that no attribute call happens during graph capture
     return cudaFuncSetAttribute(k_solver, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -609,18 +829,35 @@ int launch_bundle_ranges(const World& w, const Scratch& s, cudaStream_t st) {
     return 1;
 }
 
+// Warps per block by the largest bundle: a settled pile has about a quarter
+// contact per body, two thirds of them chained, and the warps without chained
+// contacts take the lone ones.  Solver time per substep with 1 / 2 / 4 warps:
+// 1,024 scenes in 512-body bundles 274 / 226 / 183 us (295 us before), one
+// 512-body scene - / 162 / 124 us (208 us before).  Above 512 bodies a lane pair
+// of warps more keeps a lane for every chained contact.
+static void launch_flow(const World& w, const Consts& k, const Scratch& s, uint32_t mode, float dt,
+                        uint32_t nbmax, cudaStream_t st) {
+    const uint32_t warps = nbmax <= 128 ? 1u : nbmax <= 256 ? 2u : nbmax <= 512 ? 4u : 8u;
+    // three blocks of four warps share an SM (registers): a third of its shared
+    // memory each, and records that do not fit go to global memory
+    const uint32_t budget = std::min(kFlowMaxSmem, 19456u * warps);
+    const uint32_t base = flow_smem_bytes(nbmax, 0);
+    const uint32_t recs = budget > base ? (budget - base) / (16 * kRecWords) : 0u;
+    const uint32_t smem = flow_smem_bytes(nbmax, recs);
+    switch (warps) {
+        case 1: k_solver_flow<1><<<w.nbundles, 32, smem, st>>>(w, k, s, mode, dt, nbmax, recs); break;
+        case 2: k_solver_flow<2><<<w.nbundles, 64, smem, st>>>(w, k, s, mode, dt, nbmax, recs); break;
+        case 4: k_solver_flow<4><<<w.nbundles, 128, smem, st>>>(w, k, s, mode, dt, nbmax, recs); break;
+        default: k_solver_flow<8><<<w.nbundles, 256, smem, st>>>(w, k, s, mode, dt, nbmax, recs);
+    }
+}
+
 int launch_solver(const World& w, const Consts& k, const Scratch& s, uint32_t mode, float dt,
-                  uint32_t max_scene_bodies, uint32_t smem_bodies, cudaStream_t st) {
+                  uint32_t max_scene_bodies, cudaStream_t st) {
     if (w.nbundles == 0 || w.max_contacts == 0) return 0;
     launch_bundle_ranges(w, s, st);
     if (max_scene_bodies <= kWarpMaxBodies) {
-        uint32_t nbmax = smem_bodies < max_scene_bodies ? smem_bodies : max_scene_bodies;
-        if (nbmax == 0) nbmax = 1;
-        const size_t smem = warp_smem_words(nbmax) * sizeof(float);
-        if (s.sweep_warps >= 2)
-            k_solver_warp<2><<<w.nbundles, 64, smem, st>>>(w, k, s, mode, dt, nbmax);
-        else
-            k_solver_warp<1><<<w.nbundles, 32, smem, st>>>(w, k, s, mode, dt, nbmax);
+        launch_flow(w, k, s, mode, dt, std::max(max_scene_bodies, 1u), st);
         return 2;
     }
     if (s.isl.parent) return 1 + launch_solver_islands(w, k, s, mode, dt, st);
