@@ -1347,21 +1347,20 @@ seevr_status seevr_physics_adjoint_substep(seevr_physics* h, uint32_t num_bodies
         st = dev_alloc(h, &a.tape, nc * iters * 13);
         if (st == SEEVR_OK) st = dev_alloc(h, &a.ptape, np * 2);
         if (st == SEEVR_OK) st = dev_alloc(h, &a.ctape, nc * 2);
-        if (st == SEEVR_OK) st = dev_alloc(h, &a.vw, nb * 6);
-        if (st == SEEVR_OK) st = dev_alloc(h, &a.gv, nb * 3);
-        if (st == SEEVR_OK) st = dev_alloc(h, &a.gw, nb * 3);
+        if (st == SEEVR_OK) st = dev_alloc(h, &a.side, nc);
+        if (st == SEEVR_OK) st = dev_alloc(h, &a.degree, nc);
+        if (st == SEEVR_OK) st = dev_alloc(h, &a.lam, nc);
+        if (st == SEEVR_OK) st = dev_alloc(h, &a.body4, nb * 2);
+        if (st == SEEVR_OK) st = dev_alloc(h, &a.last, nb);
+        if (st == SEEVR_OK) st = dev_alloc(h, &a.gvw, nb * 6);
         if (st == SEEVR_OK) st = dev_alloc(h, &a.gR, nb * 9);
         if (st == SEEVR_OK) st = dev_alloc(h, &a.gp, nb * 3);
         if (st == SEEVR_OK) st = dev_alloc(h, &a.gq, nb * 4);
         if (st == SEEVR_OK) st = dev_alloc(h, &a.gc, nc * 12);
         if (st == SEEVR_OK) st = dev_alloc(h, &a.glam, nc);
-        if (st == SEEVR_OK) st = dev_alloc(h, &a.lam, nc);
-        if (st == SEEVR_OK) st = dev_alloc(h, &a.par, nc * 12);
-        if (st == SEEVR_OK) st = dev_alloc(h, &a.last, nb);
-        if (st == SEEVR_OK) st = dev_alloc(h, &a.level, nc);
-        if (st == SEEVR_OK) st = dev_alloc(h, &a.order, nc);
-        if (st == SEEVR_OK) st = dev_alloc(h, &a.lvl, nc + size_t(h->caps.max_scenes) + 2);
         if (st == SEEVR_OK) st = dev_alloc(h, &a.fix, nc * 40);
+        if (st == SEEVR_OK && init_adjoint() != cudaSuccess)
+            st = fail(SEEVR_ERR_CUDA, "cudaFuncSetAttribute for the adjoint failed");
         if (st != SEEVR_OK) return st;
         h->adj_ready = true;
     }
@@ -1383,7 +1382,7 @@ seevr_status seevr_physics_adjoint_substep(seevr_physics* h, uint32_t num_bodies
     n += launch_narrowphase_taped(w, h->k, h->s, a.ptape, a.ctape, s);
     n += launch_bundle_ranges(w, h->s, s);
     const Grads g{grads->pos, grads->quat, grads->vel, grads->omega, grads->friction};
-    n += launch_adjoint(w, h->k, h->s, a, g, dt, s);
+    n += launch_adjoint(w, h->k, h->s, a, g, dt, h->max_bundle_bodies, s);
     h->launches += n;
     SEEVR_CUDA(cudaGetLastError());
     bool overflow = false;
