@@ -195,7 +195,7 @@ __device__ __forceinline__ bool update_half(const HalfRec& h, uint32_t side, f3&
     if (kBuiltin) {
         td = divs(vt, len);
     } else {
-        const float rl = recip_of(len, recip_of(len, rs));  // rs: two ulps off at worst
+        const float rl = recip_of(len, rcp_approx(len));
         td = mk(div_by(vt.x, len, rl), div_by(vt.y, len, rl), div_by(vt.z, len, rl));
     }
     const f3 rt = cross(h.r, td);
@@ -282,7 +282,7 @@ __device__ __forceinline__ bool mid_half(const HalfRec& h, uint32_t side, f3 v, 
     if (kBuiltin) {
         m.td = divs(m.vt, m.s);
     } else {
-        const float rl = recip_of(m.s, recip_of(m.s, rs));
+        const float rl = recip_of(m.s, rcp_approx(m.s));
         m.td = mk(div_by(m.vt.x, m.s, rl), div_by(m.vt.y, m.s, rl), div_by(m.vt.z, m.s, rl));
     }
     m.rt = cross(h.r, m.td);

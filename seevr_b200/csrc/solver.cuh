@@ -158,7 +158,7 @@ __device__ __forceinline__ bool update_core(const Rec& h, f3& va, f3& wa, f3& vb
     if (kBuiltin) {
         td = divs(vt, len);
     } else {
-        const float rl = recip_of(len, recip_of(len, rs));  // rs: two ulps off at worst
+        const float rl = recip_of(len, rcp_approx(len));
         td = mk(div_by(vt.x, len, rl), div_by(vt.y, len, rl), div_by(vt.z, len, rl));
     }
     const f3 rat = cross(A.r, td), rbt = cross(B.r, td);

@@ -19,7 +19,9 @@ using namespace seevr;
 __device__ unsigned next(unsigned& s) { s ^= s << 13; s ^= s >> 17; s ^= s << 5; return s; }
 __global__ void k_compare(unsigned long long* bad) {
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
-    const unsigned exps[4] = {60u, 61u, 127u, 190u};  // root: 2^-67 .. 2^63, both parities
+    // root: 2^-67 .. 2^63, both parities (a root's mantissa lies in [1, 1.41) or
+    // [1.41, 2) with the parity); reciprocals: 2^-27 .. 2^23
+    const unsigned exps[6] = {60u, 100u, 126u, 127u, 150u, 189u};
     for (unsigned m = t; m < (1u << 23); m += n)
         for (unsigned e : exps) {
             const float a = __uint_as_float((e << 23) | m);
@@ -27,7 +29,7 @@ __global__ void k_compare(unsigned long long* bad) {
             if (root_of(a, r) != root) atomicAdd(&bad[0], 1ull);
             if (e >= 90u && e <= 160u) {
                 if (recip_of(a, rcp_approx(a)) != 1.0f / a) atomicAdd(&bad[1], 1ull);
-                if (recip_of(root, recip_of(root, r)) != 1.0f / root) atomicAdd(&bad[2], 1ull);
+                if (recip_of(root, rcp_approx(root)) != 1.0f / root) atomicAdd(&bad[2], 1ull);
             }
         }
     unsigned s = 2654435761u * (t + 1u);
