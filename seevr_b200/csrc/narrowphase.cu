@@ -15,6 +15,19 @@
 // and a lane whose pair finishes takes the next pair from a global counter
 // (warp-aggregated atomics), so all lanes stay busy until the pair list is
 // exhausted and converge on the support call, the expensive part of a step.
+//
+// A step of a warp takes about 3,000 cycles whether one lane is active or all
+// (both support paths, every state's branch), and a pair's steps are one chain, so
+// with few pairs a launch is its longest chain at 3,000 cycles a step.  Up to
+// kFewPairs pairs per sixteen lanes of the grid, sixteen lanes therefore take one
+// pair together: eight per shape share the support call's candidates (one load
+// latency, then a reduction by shuffles), and the rest of the step, which all
+// sixteen compute alike, has no other pair's branches in its way: about 700 cycles.
+// Measured, a lane per pair against sixteen: 826 pairs 59 / 21 us, 10,500 pairs
+// 103 / 32 us, 26,000 pairs 95 / 61 us, 41,000 pairs 105 / 92 us; 77,000 pairs
+// 117 / 150 us, where lanes are what is short.  (Handing a warp's last eight pairs
+// to sixteen lanes each, and a pass of every pair's first two support calls before
+// the rest, changed nothing or cost up to a quarter with 115,000 pairs.)
 // The arithmetic and the order of every test are those of the reference
 // loops, so each pair's result is the same bit for bit.
 //
@@ -167,7 +180,7 @@ __device__ __forceinline__ void take(Mink& dst, const Mink& m, uint32_t& free) {
 }
 
 __device__ __forceinline__ f3 portal_dir(f3 v1, f3 v2, f3 v3) {
-    return normalize(cross(sub(v2, v1), sub(v3, v1)));
+    return normalize_fast(cross(sub(v2, v1), sub(v3, v1)));
 }
 __device__ __forceinline__ bool reach_tol(const Consts& k, f3 v1, f3 v2, f3 v3, f3 v4, f3 dir) {
     const float dv1 = dot(v1, dir), dv2 = dot(v2, dir), dv3 = dot(v3, dir), dv4 = dot(v4, dir);
@@ -234,95 +247,56 @@ __device__ __forceinline__ void finish(float4* res0, float4* res1, uint32_t* fla
 // portal (tape[2p] = {case, m1.ia, m1.ib, m2.ia}, tape[2p+1] = {m2.ib,
 // m3.ia, m3.ib, 0}; case 1 = penetration portal, 2 = the segment case of
 // physics.comp:267-271), from which the adjoint differentiates the contact.
-// kMinBlocks: resident blocks per SM the register allocation is capped for
-// (7: 72 registers with a few spilled values; 6: about 80, no spills).
-template <bool kTape, uint32_t kMinBlocks>
-__global__ void __launch_bounds__(kNarrowThreads, kMinBlocks)
-    k_narrow(World w, Consts k, float4* __restrict__ res0, float4* __restrict__ res1,
-             uint32_t* __restrict__ flag, uint32_t* __restrict__ ticket,
-             uint4* __restrict__ tape, const uint32_t* __restrict__ order) {
-    __shared__ float wit[4][Witness<kTape>::kWords][kNarrowThreadsW];
-    __shared__ float pose[2][12][kNarrowThreadsW];
-    if (halted(w.status)) return;  // pairs from a scan that gave up
-    const uint32_t np = min(w.counters[0], w.max_pairs);
-    const uint32_t lane = threadIdx.x & 31u;
-    const unsigned full = 0xFFFFFFFFu;
-    const Witness<kTape> W{wit, threadIdx.x};
-    const Pose P{pose, threadIdx.x};
+struct Out {
+    float4* res0;
+    float4* res1;
+    uint32_t* flag;
+    uint4* tape;
+};
 
-    bool active = false, drained = false;
-    uint32_t p = 0, state = kD1, iter = 0;
-    Shape A, B;
-    f3 v0 = mk(0, 0, 0), dir = mk(0, 0, 0);
-    Mink m1{mk(0, 0, 0), 0}, m2{mk(0, 0, 0), 1}, m3{mk(0, 0, 0), 2};
-    uint32_t free = 3;
+// The state of one pair's MPR.
+struct Mpr {
+    uint32_t p, state, iter, free;
+    f3 v0, dir;
+    Mink m1, m2, m3;
 
-    while (true) {
-        // ---- refill idle lanes with the next pairs ----
-        if (!drained) {
-            const unsigned need = __ballot_sync(full, !active);
-            if (need) {
-                const uint32_t leader = __ffs(need) - 1;
-                uint32_t base = 0;
-                if (lane == leader) base = atomicAdd(ticket, uint32_t(__popc(need)));
-                base = __shfl_sync(full, base, leader);
-                if (base + __popc(need) >= np) drained = true;
-                if (!active) {
-                    const uint32_t q = base + __popc(need & ((1u << lane) - 1u));
-                    if (q < np) {
-                        p = order ? order[q] : q;
-                        const uint32_t a = w.pairs[size_t(p) * 2], b = w.pairs[size_t(p) * 2 + 1];
-                        A = load_shape(w, a, P, 0);
-                        B = load_shape(w, b, P, 1);
-                        v0 = sub(ld3(w.pos, a), ld3(w.pos, b));  // s0a - s0b (physics.comp:254-258)
-                        if (fabsf(v0.x) < k.eps && fabsf(v0.y) < k.eps && fabsf(v0.z) < k.eps)
-                            v0.x += 10.0f * k.eps;
-                        dir = normalize(neg(v0));
-                        state = kD1;
-                        iter = 0;
-                        active = true;
-                    }
-                }
-            }
-        }
-        if (__ballot_sync(full, active) == 0u) break;
-        if (!active) continue;
-
-        // ---- prelude: the direction of this step's support call ----
+    __device__ __forceinline__ void start(const Consts& k, uint32_t pair, f3 c) {
+        p = pair;
+        v0 = c;  // s0a - s0b (physics.comp:254-258)
+        if (fabsf(v0.x) < k.eps && fabsf(v0.y) < k.eps && fabsf(v0.z) < k.eps)
+            v0.x += 10.0f * k.eps;
+        dir = normalize_fast(neg(v0));
+        state = kD1;
+        iter = 0;
+    }
+    // No contact.
+    __device__ __forceinline__ bool miss(const Out& o, bool write) const {
+        if (write) finish(o.res0, o.res1, o.flag, p, false, v0, v0, 0.0f);
+        return false;
+    }
+    // The direction of this step's support call; false when the pair is done.
+    // write: this lane records the pair's outcome.
+    __device__ __forceinline__ bool before(const Consts& k, const Out& o, bool write) {
         if (state == kR) {
             dir = portal_dir(m1.v, m2.v, m3.v);
             if (dot(m1.v, dir) > -k.eps) {  // origin inside: refine returns 0
                 state = kP;
                 iter = 0;
-                if (k.mpr_iterations == 0) {
-                    finish(res0, res1, flag, p, false, v0, v0, 0.0f);
-                    active = false;
-                    continue;
-                }
+                if (k.mpr_iterations == 0) return miss(o, write);
             }
         } else if (state == kP) {
             dir = portal_dir(m1.v, m2.v, m3.v);
         }
-
-        // ---- the one Minkowski support call of the step ----
-        Mink m;
-        {
-            uint32_t ia, ib;
-            const f3 sa = support(w, A, P, 0, dir, ia);
-            const f3 sb = support(w, B, P, 1, neg(dir), ib);
-            m.v = sub(sa, sb);
-            m.slot = free;
-            W.put(free, sa, sb, ia, ib);
-        }
-
-        // ---- postlude ----
+        return true;
+    }
+    // Takes the support point m (held in slot `free`) along dir; false when the
+    // pair is done.
+    template <bool kTape>
+    __device__ __forceinline__ bool after(const Consts& k, const Out& o, bool write, const Mink& m,
+                                          const Witness<kTape>& W, const Pose& P) {
         switch (state) {
             case kD1: {
-                if (dot(m.v, dir) < k.eps) {
-                    finish(res0, res1, flag, p, false, v0, v0, 0.0f);
-                    active = false;
-                    break;
-                }
+                if (dot(m.v, dir) < k.eps) return miss(o, write);
                 take(m1, m, free);
                 const f3 c = cross(v0, m1.v);
                 if (dot(c, c) < k.eps) {
@@ -336,27 +310,24 @@ __global__ void __launch_bounds__(kNarrowThreads, kMinBlocks)
                         depth = length(v1);  // origin on segment v0-v1: res == 2
                         n = normalize(v1);
                     }
-                    if (kTape) {
-                        tape[size_t(p) * 2] = make_uint4(2u, W.ia(m1.slot), W.ib(m1.slot), 0u);
-                        tape[size_t(p) * 2 + 1] = make_uint4(0u, 0u, 0u, 0u);
+                    if (write) {
+                        if (kTape) {
+                            o.tape[size_t(p) * 2] = make_uint4(2u, W.ia(m1.slot), W.ib(m1.slot), 0u);
+                            o.tape[size_t(p) * 2 + 1] = make_uint4(0u, 0u, 0u, 0u);
+                        }
+                        finish(o.res0, o.res1, o.flag, p, true,
+                               scale(0.5f, add(W.sa(m1.slot), W.sb(m1.slot))), n, depth);
                     }
-                    finish(res0, res1, flag, p, true,
-                           scale(0.5f, add(W.sa(m1.slot), W.sb(m1.slot))), n, depth);
-                    active = false;
-                    break;
+                    return false;
                 }
-                dir = normalize(c);
+                dir = normalize_fast(c);
                 state = kD2;
-                break;
+                return true;
             }
             case kD2: {
-                if (dot(m.v, dir) < k.eps) {
-                    finish(res0, res1, flag, p, false, v0, v0, 0.0f);
-                    active = false;
-                    break;
-                }
+                if (dot(m.v, dir) < k.eps) return miss(o, write);
                 take(m2, m, free);
-                dir = normalize(cross(sub(m1.v, v0), sub(m2.v, v0)));
+                dir = normalize_fast(cross(sub(m1.v, v0), sub(m2.v, v0)));
                 if (dot(dir, v0) > 0.0f) {
                     const Mink t = m1;
                     m1 = m2;
@@ -365,18 +336,10 @@ __global__ void __launch_bounds__(kNarrowThreads, kMinBlocks)
                 }
                 iter = 0;  // discovery trials
                 state = kDT;
-                if (k.discover_trials == 0) {
-                    finish(res0, res1, flag, p, false, v0, v0, 0.0f);
-                    active = false;
-                }
-                break;
+                return k.discover_trials == 0 ? miss(o, write) : true;
             }
             case kDT: {
-                if (dot(m.v, dir) < k.eps) {
-                    finish(res0, res1, flag, p, false, v0, v0, 0.0f);
-                    active = false;
-                    break;
-                }
+                if (dot(m.v, dir) < k.eps) return miss(o, write);
                 bool retry = false;
                 if (dot(cross(m1.v, m.v), v0) < -k.eps) {
                     take(m2, m, free);
@@ -386,54 +349,209 @@ __global__ void __launch_bounds__(kNarrowThreads, kMinBlocks)
                     retry = true;
                 }
                 if (retry) {
-                    dir = normalize(cross(sub(m1.v, v0), sub(m2.v, v0)));
-                    if (++iter >= k.discover_trials) {
-                        finish(res0, res1, flag, p, false, v0, v0, 0.0f);
-                        active = false;
-                    }
-                    break;
+                    dir = normalize_fast(cross(sub(m1.v, v0), sub(m2.v, v0)));
+                    return ++iter >= k.discover_trials ? miss(o, write) : true;
                 }
                 take(m3, m, free);  // portal found: refine
                 iter = 0;
                 state = kR;
-                if (k.mpr_iterations == 0) {  // refine returns 1, penetration finds nothing
-                    finish(res0, res1, flag, p, false, v0, v0, 0.0f);
-                    active = false;
-                }
-                break;
+                // no iterations: refine returns 1, penetration finds nothing
+                return k.mpr_iterations == 0 ? miss(o, write) : true;
             }
             case kR: {
-                if (!(dot(m.v, dir) > -k.eps) || reach_tol(k, m1.v, m2.v, m3.v, m.v, dir)) {
-                    finish(res0, res1, flag, p, false, v0, v0, 0.0f);
-                    active = false;
-                    break;
-                }
+                if (!(dot(m.v, dir) > -k.eps) || reach_tol(k, m1.v, m2.v, m3.v, m.v, dir))
+                    return miss(o, write);
                 expand(v0, m1, m2, m3, m, free);
                 if (++iter >= k.mpr_iterations) {  // refine returns 1: go on to penetration
                     iter = 0;
                     state = kP;
                 }
-                break;
+                return true;
             }
             default: {  // kP
                 if (reach_tol(k, m1.v, m2.v, m3.v, m.v, dir) || iter >= k.mpr_iterations - 1) {
-                    const float depth = dot(dir, m1.v);
-                    if (kTape) {
-                        tape[size_t(p) * 2] =
-                            make_uint4(1u, W.ia(m1.slot), W.ib(m1.slot), W.ia(m2.slot));
-                        tape[size_t(p) * 2 + 1] =
-                            make_uint4(W.ib(m2.slot), W.ia(m3.slot), W.ib(m3.slot), 0u);
+                    if (write) {
+                        const float depth = dot(dir, m1.v);
+                        if (kTape) {
+                            o.tape[size_t(p) * 2] =
+                                make_uint4(1u, W.ia(m1.slot), W.ib(m1.slot), W.ia(m2.slot));
+                            o.tape[size_t(p) * 2 + 1] =
+                                make_uint4(W.ib(m2.slot), W.ia(m3.slot), W.ib(m3.slot), 0u);
+                        }
+                        finish(o.res0, o.res1, o.flag, p, true,
+                               find_pos(k, v0, P.p(0), P.p(1), m1, m2, m3, W), dir, depth);
                     }
-                    finish(res0, res1, flag, p, true,
-                           find_pos(k, v0, P.p(0), P.p(1), m1, m2, m3, W), dir, depth);
-                    active = false;
-                    break;
+                    return false;
                 }
                 expand(v0, m1, m2, m3, m, free);
                 ++iter;
-                break;
+                return true;
             }
         }
+    }
+};
+
+// The support point of the calling lane's shape along its d, found by the eight
+// lanes of the shape (half: the sixteen lanes of the pair): each takes every eighth
+// candidate of the reference's order, and the first strict maximum is the greatest
+// value at the lowest place.
+__device__ __forceinline__ f3 support_shared(const World& w, const Shape& s, const m3& R, f3 pos,
+                                             f3 d, unsigned half, uint32_t& chosen) {
+    const uint32_t l8 = threadIdx.x & 7u;
+    const f3 ld = mulT(R, d);
+    float best = -1e10f;
+    f3 bv = mk(0.f, 0.f, 0.f);
+    uint32_t place = kNone, idx = kNone;
+    if (s.lk != 0u) {
+        if (l8 < 6u) {  // the angle bins of the X, Y, Z axes, two candidates each
+            const uint32_t ax = l8 >> 1;
+            const uint32_t b = angle_bin64(ax == 2u ? ld.y : ld.z, ax == 0u ? ld.y : ld.x);
+            idx = w.sup_lut[s.lk + ax * 64u + ((b + (l8 & 1u)) & 63u)];
+            const f3 v = ld3(w.hull, s.vs + idx);
+            const float dd = dot(v, ld);
+            if (dd > best) {
+                best = dd;
+                bv = v;
+                place = l8;
+            }
+        }
+    } else {
+        for (uint32_t k = l8; k < s.vc; k += 8u) {
+            const f3 v = ld3(w.hull, s.vs + k);
+            const float dd = dot(v, ld);
+            if (dd > best) {
+                best = dd;
+                bv = v;
+                place = idx = k;
+            }
+        }
+    }
+    __syncwarp(half);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        const float ob = __shfl_xor_sync(half, best, o);
+        const uint32_t op = __shfl_xor_sync(half, place, o);
+        if (ob > best || (ob == best && op < place)) {
+            best = ob;
+            place = op;
+        }
+    }
+    // the winner's lane holds its vertex (none: every lane holds zero)
+    const uint32_t src = (threadIdx.x & 24u) | (place & 7u);
+    bv = mk(__shfl_sync(half, bv.x, src), __shfl_sync(half, bv.y, src), __shfl_sync(half, bv.z, src));
+    idx = __shfl_sync(half, idx, src);
+    chosen = place == kNone ? kNone : idx;
+    return add(pos, mul(R, bv));
+}
+
+// Pairs per sixteen lanes up to which sixteen lanes take a pair together.
+constexpr uint32_t kFewPairs = 6;
+
+// kMinBlocks: resident blocks per SM the register allocation is capped for
+// (7: 72 registers with a few spilled values; 6: about 80).
+template <bool kTape, uint32_t kMinBlocks>
+__global__ void __launch_bounds__(kNarrowThreads, kMinBlocks)
+    k_narrow(World w, Consts k, Out o, uint32_t* __restrict__ ticket,
+             const uint32_t* __restrict__ order) {
+    __shared__ float wit[4][Witness<kTape>::kWords][kNarrowThreadsW];
+    __shared__ float pose[2][12][kNarrowThreadsW];
+    if (halted(w.status)) return;  // pairs from a scan that gave up
+    const uint32_t np = min(w.counters[0], w.max_pairs);
+    const uint32_t lane = threadIdx.x & 31u;
+    const unsigned full = 0xFFFFFFFFu;
+    if (np > gridDim.x * (kNarrowThreads / 16u) * kFewPairs) {  // ---- a lane per pair ----
+        const Witness<kTape> W{wit, threadIdx.x};
+        const Pose P{pose, threadIdx.x};
+        bool active = false, drained = false;
+        Shape A{}, B{};
+        Mpr q{};
+        q.m1.slot = 0;
+        q.m2.slot = 1;
+        q.m3.slot = 2;
+        q.free = 3;
+        while (true) {
+            // ---- refill idle lanes with the next pairs ----
+            if (!drained) {
+                const unsigned need = __ballot_sync(full, !active);
+                if (need) {
+                    const uint32_t leader = __ffs(need) - 1;
+                    uint32_t base = 0;
+                    if (lane == leader) base = atomicAdd(ticket, uint32_t(__popc(need)));
+                    base = __shfl_sync(full, base, leader);
+                    if (base + __popc(need) >= np) drained = true;
+                    if (!active) {
+                        const uint32_t i = base + __popc(need & ((1u << lane) - 1u));
+                        if (i < np) {
+                            const uint32_t p = order ? order[i] : i;
+                            const uint32_t a = w.pairs[size_t(p) * 2], b = w.pairs[size_t(p) * 2 + 1];
+                            A = load_shape(w, a, P, 0);
+                            B = load_shape(w, b, P, 1);
+                            q.start(k, p, sub(ld3(w.pos, a), ld3(w.pos, b)));
+                            active = true;
+                        }
+                    }
+                }
+            }
+            if (__ballot_sync(full, active) == 0u) break;
+            if (!active) continue;
+            active = q.before(k, o, true);
+            if (!active) continue;
+            // ---- the one Minkowski support call of the step ----
+            Mink m;
+            {
+                uint32_t ia, ib;
+                const f3 sa = support(w, A, P, 0, q.dir, ia);
+                const f3 sb = support(w, B, P, 1, neg(q.dir), ib);
+                m.v = sub(sa, sb);
+                m.slot = q.free;
+                W.put(q.free, sa, sb, ia, ib);
+            }
+            active = q.after(k, o, true, m, W, P);
+        }
+        return;
+    }
+
+    // ---- sixteen lanes per pair: lanes 0-7 shape A, 8-15 shape B ----
+    const unsigned half = lane < 16u ? 0x0000FFFFu : 0xFFFF0000u;
+    const uint32_t first = lane & 16u, side = (lane >> 3) & 1u;
+    const bool writes = (lane & 15u) == 0u;
+    const uint32_t t = (threadIdx.x & ~31u) | first;  // the thread whose pose and witness slots they use
+    const Witness<kTape> W{wit, t};
+    const Pose P{pose, t};
+    for (;;) {
+        uint32_t i = 0;
+        if (writes) i = atomicAdd(ticket, 1u);
+        i = __shfl_sync(half, i, first);
+        if (i >= np) return;
+        const uint32_t p = order ? order[i] : i;
+        const uint32_t a = w.pairs[size_t(p) * 2], b = w.pairs[size_t(p) * 2 + 1];
+        const uint32_t body = side ? b : a;
+        Shape S;
+        if ((lane & 7u) == 0u) S = load_shape(w, body, P, side);
+        else S = Shape{w.hull_range[size_t(body) * 2], w.hull_range[size_t(body) * 2 + 1], lut_of(w, body)};
+        Mpr q;
+        q.m1.slot = 0;
+        q.m2.slot = 1;
+        q.m3.slot = 2;
+        q.free = 3;
+        q.start(k, p, sub(ld3(w.pos, a), ld3(w.pos, b)));
+        __syncwarp(half);
+        const m3 R = P.R(side);
+        const f3 pos = P.p(side);
+        while (q.before(k, o, writes)) {
+            uint32_t mine;
+            const f3 pt = support_shared(w, S, R, pos, side ? neg(q.dir) : q.dir, half, mine);
+            const f3 other = mk(__shfl_xor_sync(half, pt.x, 8), __shfl_xor_sync(half, pt.y, 8),
+                                __shfl_xor_sync(half, pt.z, 8));
+            const uint32_t theirs = __shfl_xor_sync(half, mine, 8);
+            const f3 sa = side ? other : pt, sb = side ? pt : other;
+            Mink m;
+            m.v = sub(sa, sb);
+            m.slot = q.free;
+            if (writes) W.put(q.free, sa, sb, mine, theirs);
+            if (!q.after(k, o, writes, m, W, P)) break;
+        }
+        __syncwarp(half);  // the pair's poses are read
     }
 }
 
@@ -813,8 +931,10 @@ int launch_narrowphase_taped(const World& w, const Consts& k, const Scratch& s, 
     // persistent grid: a few resident blocks per SM; the pair ticket lives
     // in status[1] and is cleared here
     cudaMemsetAsync(&s.status[1], 0, sizeof(uint32_t), st);
-    const uint32_t blocks = grid_for(w.max_pairs, kNarrowThreads,
-                                     s.narrow_blocks ? s.narrow_blocks : 148 * kNarrowBlocksPerSm);
+    // (four lanes per pair that the buffers can hold, so that few pairs get
+    // sixteen each)
+    const uint32_t most = s.narrow_blocks ? s.narrow_blocks : 148 * kNarrowBlocksPerSm;
+    const uint32_t blocks = grid_for(w.max_pairs, kNarrowThreads / 4, most);
     // the register budget of seven blocks per SM when that many are resident,
     // else the larger one of six
     const bool seven = (s.narrow_per_sm ? s.narrow_per_sm : kNarrowBlocksPerSm) >= 7;
@@ -832,20 +952,13 @@ int launch_narrowphase_taped(const World& w, const Consts& k, const Scratch& s, 
     if (k.narrowphase == 1u && !pair_tape) {  // GJK + EPA (the adjoint tapes MPR only)
         k_gjk_epa<<<grid_for(w.max_pairs, 128, uint32_t(148 * 16)), 128, 0, st>>>(
             w, k, s.pair_res0, s.pair_res1, s.pair_flag, order);
-    } else if (pair_tape) {
-        if (seven)
-            k_narrow<true, 7><<<blocks, kNarrowThreads, 0, st>>>(
-                w, k, s.pair_res0, s.pair_res1, s.pair_flag, &s.status[1], pair_tape, order);
-        else
-            k_narrow<true, 6><<<blocks, kNarrowThreads, 0, st>>>(
-                w, k, s.pair_res0, s.pair_res1, s.pair_flag, &s.status[1], pair_tape, order);
     } else {
-        if (seven)
-            k_narrow<false, 7><<<blocks, kNarrowThreads, 0, st>>>(
-                w, k, s.pair_res0, s.pair_res1, s.pair_flag, &s.status[1], nullptr, order);
-        else
-            k_narrow<false, 6><<<blocks, kNarrowThreads, 0, st>>>(
-                w, k, s.pair_res0, s.pair_res1, s.pair_flag, &s.status[1], nullptr, order);
+        const Out o{s.pair_res0, s.pair_res1, s.pair_flag, pair_tape};
+        uint32_t* ticket = &s.status[1];
+        if (pair_tape && seven) k_narrow<true, 7><<<blocks, kNarrowThreads, 0, st>>>(w, k, o, ticket, order);
+        else if (pair_tape) k_narrow<true, 6><<<blocks, kNarrowThreads, 0, st>>>(w, k, o, ticket, order);
+        else if (seven) k_narrow<false, 7><<<blocks, kNarrowThreads, 0, st>>>(w, k, o, ticket, order);
+        else k_narrow<false, 6><<<blocks, kNarrowThreads, 0, st>>>(w, k, o, ticket, order);
     }
     launch_exclusive_scan(s.pair_flag, s.pair_coff, &w.counters[0], w.max_pairs,
                           &w.counters[1], w.max_contacts, kFlagContactOverflow, s, st);
