@@ -5,11 +5,13 @@
 // its own kernel after the state update.
 //
 // The stage streams every hull vertex once per substep (12 bytes each, the
-// bulk of its HBM traffic).  A block takes 256 consecutive bodies: each
+// bulk of its HBM traffic).  A block takes up to 256 consecutive bodies: each
 // thread updates its body's state with coalesced loads and handles a small
 // hull itself; bodies whose hull has more than 32 vertices go to a
 // per-block queue that the block's warps then drain, lanes striding over
-// the vertices, so no warp waits on a single lane's state update.
+// the vertices, so no warp waits on a single lane's state update.  A warp takes
+// about a microsecond per large hull, one after another, so few bodies are
+// spread over blocks of fewer each (launch_body_stage).
 //
 // The reference reduces AABBs with a thread-0 serial loop per 256-vertex
 // workgroup and a multi-launch cascade; min/max are exact in any order, so
@@ -131,7 +133,7 @@ __device__ __forceinline__ void body_state(const World& w, const Consts& k, uint
 // vertices and reduce with shuffles (min/max are exact in any order).
 __global__ void __launch_bounds__(kBodyThreads) k_body_stage(World w, Consts k, uint32_t flags,
                                                              float dt, float gx, float gy,
-                                                             float gz) {
+                                                             float gz, uint32_t per_block) {
     __shared__ float sh_pose[kBodyThreads][12];  // p xyz, R by columns
     __shared__ uint32_t sh_body[kBodyThreads];
     __shared__ uint32_t sh_n;
@@ -139,9 +141,9 @@ __global__ void __launch_bounds__(kBodyThreads) k_body_stage(World w, Consts k, 
     if (threadIdx.x == 0) sh_n = 0;
     __syncthreads();
 
-    const uint32_t b = blockIdx.x * kBodyThreads + threadIdx.x;
+    const uint32_t b = blockIdx.x * per_block + threadIdx.x;
     const float inf = __int_as_float(0x7f800000);
-    if (b < w.nb) {
+    if (threadIdx.x < per_block && b < w.nb) {
         uint32_t hs = 0, hc = 0;
         if (flags & kAabb) {
             hs = w.hull_range[size_t(b) * 2];
@@ -270,11 +272,16 @@ __global__ void __launch_bounds__(kRenderThreads) k_render_verts(World w) {
 int launch_body_stage(const World& w, const Consts& k, uint32_t flags, float dt, float gx,
                       float gy, float gz, cudaStream_t st) {
     if (w.nb == 0) return 0;
-    const uint32_t blocks = (w.nb + kBodyThreads - 1) / kBodyThreads;
+    // as many bodies per block as leave every SM its four blocks, at least one
+    // large hull per warp (3,491 bodies, half of them large hulls: 21 us with 256
+    // per block, 5 us with 8; 32,769 bodies: 24 us with 256, 15 us with 56)
+    uint32_t per = (w.nb + 148u * 4u - 1u) / (148u * 4u);
+    per = min(max((per + 7u) & ~7u, 8u), kBodyThreads);
+    const uint32_t blocks = (w.nb + per - 1) / per;
     // render vertices in their own kernel, after the state update: the
     // per-body stage keeps its register budget (and occupancy) for the
     // substep launches
-    k_body_stage<<<blocks, kBodyThreads, 0, st>>>(w, k, flags & ~kRenderVerts, dt, gx, gy, gz);
+    k_body_stage<<<blocks, kBodyThreads, 0, st>>>(w, k, flags & ~kRenderVerts, dt, gx, gy, gz, per);
     if (!(flags & kRenderVerts)) return 1;
     const uint32_t rblocks = (w.nb + kRenderThreads / 32 - 1) / (kRenderThreads / 32);
     k_render_verts<<<rblocks < 148u * 64u ? rblocks : 148u * 64u, kRenderThreads, 0, st>>>(w);
