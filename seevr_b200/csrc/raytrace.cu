@@ -12,16 +12,27 @@
 //     loads) and the triangles into 48-byte records in leaf order (v0 and
 //     the two edges the intersection test forms, with the triangle index),
 //     so a leaf's triangles are one contiguous read;
-//   - a persistent grid of lanes runs sample paths one bounce per loop
-//     step, and a lane whose path ends takes the next (pixel, sample) from
-//     a warp-aggregated ticket, so lanes do not idle while the longest path
-//     of their warp finishes;
+//   - the binary tree is collapsed into wide nodes of four children (each node's
+//     grandchildren, in the shader's visiting order), a 128-byte record per visit:
+//     half the dependent fetches of a path to a leaf, and no fetch for the leaf;
+//   - a persistent grid of lanes runs sample paths; a lane whose path ends takes
+//     the next (pixel, sample) from a warp-aggregated ticket.  A warp's lanes step
+//     through their trees together, and those whose ray is done wait until enough
+//     do (kShadeLanes) for their hits to be shaded together, so a warp neither
+//     waits for its longest ray nor shades one hit at a time;
 //   - each path's colour is stored per sample and a resolve pass sums a
 //     pixel's 16 samples in sample order, as the shader's loop does.
-// The traversal visits nodes in the shader's order (left pushed before
-// right, the same stack bound), every expression keeps its evaluation
-// order and the library is built without FMA contraction, so the image
-// equals the CPU restatement's bit for bit.  Three functions whose GLSL
+// Leaves are visited in the shader's order (left pushed before right), every
+// expression keeps its evaluation order and the library is built without FMA
+// contraction, so the image equals the CPU restatement's bit for bit.  (The
+// shader reaches a leaf if every box on its path is hit nearer than the closest
+// hit so far.  A child's box lies in its parent's, so by monotone rounding its
+// entry is no nearer and its exit no farther, and the closest hit only comes
+// nearer: the leaf's own box, tested when its turn comes, decides alone.  Where
+// that does not hold, the shader's own traversal of the binary tree runs: for a
+// tree whose boxes do not nest or are not finite or that overruns the shader's
+// stack (k_rt_check), and for rays with a component of zero or
+// NaN.)  Three functions whose GLSL
 // precision is implementation-defined are pinned here, and the restatement
 // uses the same definitions:
 //   - sin/cos of the hemisphere angle: reduction by quadrant (pi/2 split in
@@ -208,6 +219,137 @@ __device__ void trace(const NodeP* __restrict__ nodes, const TriP* __restrict__ 
     }
 }
 
+// ---- wide nodes ----------------------------------------------------------------
+// The four grandchildren of a node in visiting order (the right child's right, the
+// right child's left, ...; a leaf child counts as one), bounds by axis.  id: an
+// inner node, kLeafBit | the slot of a one-triangle leaf, kMulti | the node of a leaf
+// with another count, or kNone.
+struct Wide {
+    float4 lx, ly, lz, hx, hy, hz;
+    uint4 id;
+    uint4 pad;
+};
+static_assert(sizeof(Wide) == 128, "one record, four sectors");
+constexpr uint32_t kMulti = 0x40000000u, kNodeMask = 0x3FFFFFFFu;
+// The shader's stack holds the left siblings of a path's right turns and drops what
+// comes after 31 entries: nothing, if no inner node lies more right turns deep than
+constexpr uint32_t kMaxRights = 29;
+constexpr uint32_t kMaxDepth = 48;  // of a leaf, by the stack below
+constexpr int kWideStack = 3 * (kMaxDepth / 2) + 4;  // three entries a level, four being written
+
+// parent[child] = node (cleared to kNone before); *bad is raised for a tree that is
+// not one: a child out of range or with two parents.
+__global__ void k_rt_parents(RtArgs g, uint32_t nnodes, uint32_t* __restrict__ parent,
+                             uint32_t* __restrict__ bad) {
+    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < nnodes; n += gridDim.x * blockDim.x) {
+        if (g.count[n] > 0) continue;
+        const uint32_t c[2] = {g.left[n], g.right[n]};
+        for (uint32_t q = 0; q < 2; ++q)
+            if (c[q] >= nnodes || atomicExch(&parent[c[q]], n) != kNone) *bad = 1u;
+    }
+}
+
+// Raises *bad unless every node reached has finite bounds inside its parent's and a
+// place within the depths above.
+__global__ void k_rt_check(RtArgs g, const NodeP* __restrict__ nodes, uint32_t nnodes,
+                           const uint32_t* __restrict__ parent, uint32_t* __restrict__ bad) {
+    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < nnodes; n += gridDim.x * blockDim.x) {
+        const float4 lo = nodes[n].lo, hi = nodes[n].hi;
+        const uint32_t p = parent[n];
+        if (p == kNone && n != 0) continue;  // not reached from the root
+        // (a difference of equal infinities or with a NaN is NaN)
+        const float f = (lo.x - lo.x) + (lo.y - lo.y) + (lo.z - lo.z) + (hi.x - hi.x) +
+                        (hi.y - hi.y) + (hi.z - hi.z);
+        bool ok = f == 0.0f && g.count[n] < kMulti && (n != 0 || p == kNone);
+        if (p != kNone && p < nnodes) {
+            const float4 pl = nodes[p].lo, ph = nodes[p].hi;
+            ok = ok && pl.x <= lo.x && pl.y <= lo.y && pl.z <= lo.z && ph.x >= hi.x &&
+                 ph.y >= hi.y && ph.z >= hi.z;
+        }
+        if (g.count[n] > 0) {  // a leaf: the way up
+            uint32_t depth = 0, rights = 0;
+            for (uint32_t q = p, c = kNone; q != kNone && q < nnodes && depth <= kMaxDepth;
+                 c = q, q = parent[q]) {
+                ++depth;
+                rights += c != kNone && g.right[q] == c;  // the edge to an inner node
+            }
+            ok = ok && depth <= kMaxDepth && rights <= kMaxRights;
+        }
+        if (!ok) *bad = 1u;
+    }
+}
+
+__global__ void k_rt_wide(RtArgs g, const NodeP* __restrict__ nodes, uint32_t nnodes,
+                          const uint32_t* __restrict__ bad, Wide* __restrict__ out) {
+    if (*bad) return;
+    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < nnodes; n += gridDim.x * blockDim.x) {
+        if (g.count[n] > 0) continue;
+        uint32_t id[4] = {kNone, kNone, kNone, kNone};
+        float b[6][4] = {};
+        uint32_t at = 0;
+        auto put = [&](uint32_t c) {
+            const float4 lo = nodes[c].lo, hi = nodes[c].hi;
+            const uint32_t cnt = g.count[c];
+            id[at] = cnt == 1u ? kLeafBit | __float_as_uint(lo.w) : cnt > 1u ? kMulti | c : c;
+            b[0][at] = lo.x; b[1][at] = lo.y; b[2][at] = lo.z;
+            b[3][at] = hi.x; b[4][at] = hi.y; b[5][at] = hi.z;
+            ++at;
+        };
+        const uint32_t kids[2] = {g.right[n], g.left[n]};  // right first: it is on top of the stack
+        for (uint32_t q = 0; q < 2; ++q) {
+            const uint32_t c = kids[q];
+            if (g.count[c] > 0) {
+                put(c);
+            } else {
+                put(g.right[c]);
+                put(g.left[c]);
+            }
+        }
+        Wide w;
+        w.lx = make_float4(b[0][0], b[0][1], b[0][2], b[0][3]);
+        w.ly = make_float4(b[1][0], b[1][1], b[1][2], b[1][3]);
+        w.lz = make_float4(b[2][0], b[2][1], b[2][2], b[2][3]);
+        w.hx = make_float4(b[3][0], b[3][1], b[3][2], b[3][3]);
+        w.hy = make_float4(b[4][0], b[4][1], b[4][2], b[4][3]);
+        w.hz = make_float4(b[5][0], b[5][1], b[5][2], b[5][3]);
+        w.id = make_uint4(id[0], id[1], id[2], id[3]);
+        w.pad = make_uint4(0u, 0u, 0u, 0u);
+        out[n] = w;
+    }
+}
+
+// A ray's closest hit so far.
+struct Hit {
+    float t;
+    f3 normal;
+    uint32_t tri;
+    bool front;
+};
+__device__ __forceinline__ void hit_triangle(const TriP* __restrict__ tris, uint32_t slot, f3 ro,
+                                             f3 rd, Hit& h) {
+    const float4 a = __ldg(&tris[slot].a), b = __ldg(&tris[slot].b), c = __ldg(&tris[slot].c);
+    const f3 e1 = mk(b.x, b.y, b.z), e2 = mk(c.x, c.y, c.z);
+    const float t = ray_tri(ro, rd, mk(a.x, a.y, a.z), e1, e2);
+    if (t > 0.0f && t < h.t) {
+        h.t = t;
+        const f3 n = normalize(cross(e1, e2));
+        h.front = dot(n, rd) < 0.0f;
+        h.normal = h.front ? n : neg(n);
+        h.tri = __float_as_uint(a.w);
+    }
+}
+// ray_aabb's test but for the closest hit; the entry.  (Finite operands: fminf and
+// fmaxf give GLSL's min and max but for the sign of a zero.)
+__device__ __forceinline__ bool enters(f3 ro, f3 inv, float lx, float ly, float lz, float hx, float hy,
+                                       float hz, float& enter) {
+    const float ax = (lx - ro.x) * inv.x, bx = (hx - ro.x) * inv.x;
+    const float ay = (ly - ro.y) * inv.y, by = (hy - ro.y) * inv.y;
+    const float az = (lz - ro.z) * inv.z, bz = (hz - ro.z) * inv.z;
+    enter = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fminf(az, bz));
+    const float exit_ = fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz));
+    return exit_ >= enter && exit_ > 0.0f;
+}
+
 __device__ __forceinline__ f3 sky_color(f3 rd) {  // raytrace.comp:135-138
     const float t = 0.5f * (rd.y + 1.0f);
     return scale(0.8f, mix3(mk(1.f, 1.f, 1.f), mk(0.5f, 0.7f, 1.0f), t));
@@ -231,6 +373,13 @@ __device__ __forceinline__ float schlick(float cos_theta, float r0) {  // 157-15
 }
 
 constexpr uint32_t kRtThreads = 128;
+// Lanes of a warp whose ray is done at which their hits are shaded, and lanes at inner
+// nodes up to which a warp goes on to the leaves.  A frame is bound by issue (68% of
+// the slots) with few lanes active per instruction (6 of 32 before), so both are
+// chosen for full warps: 640x480 over 134,156 triangles 6.28 ms (9.86 ms with the
+// binary tree one bounce per step); 7.0 ms with 6 and 4, 7.9 ms with 20 and 0.
+constexpr int kShadeLanes = 20;
+constexpr int kInnerLanes = 10;
 
 // The camera ray of sample si of pixel (px, py) (raytrace.comp:176-190).
 __device__ __forceinline__ void camera_ray(const RtArgs& g, uint32_t px, uint32_t py, uint32_t si,
@@ -245,29 +394,74 @@ __device__ __forceinline__ void camera_ray(const RtArgs& g, uint32_t px, uint32_
     ro = g.cam_pos;
 }
 
-// Sample paths (raytrace.comp:192-270), one bounce per loop step.  Item q
+// Sample paths (raytrace.comp:192-270).  Item q
 // is sample q % 16 of pixel q / 16 (row-major), so a warp's first paths are
 // two neighbouring pixels' samples; its colour goes to samples[3q..3q+2].
 __global__ void __launch_bounds__(kRtThreads) k_rt_paths(RtArgs g, const NodeP* __restrict__ nodes,
+                                                         const Wide* __restrict__ wide,
                                                          const TriP* __restrict__ tris,
                                                          float* __restrict__ samples,
                                                          uint32_t* __restrict__ ticket,
+                                                         const uint32_t* __restrict__ bad,
                                                          uint32_t nitems) {
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned full = 0xFFFFFFFFu;
-    bool active = false, drained = false;
+    const bool plain = *bad != 0u;  // only the shader's own traversal
+    enum : uint32_t { kIdle, kTracing, kWaiting };
+    uint32_t mode = kIdle;
+    bool drained = false;
     uint32_t item = 0, seed = 0, bounce = 0;
-    f3 ro = mk(0.f, 0.f, 0.f), rd = ro, throughput = ro, color = ro;
+    f3 ro = mk(0.f, 0.f, 0.f), rd = ro, inv = ro, throughput = ro, color = ro;
+    Hit h{};
+    uint2 stack[kWideStack];  // node or leaf, bits of its entry
+    int sp = 0;
+    uint32_t cur = kNone;  // the node or leaf the lane is at
+    // Pushes the children of the inner node cur that the ray enters, last to first, so
+    // that the first is on top.
+    auto visit = [&] {
+        const Wide* w = wide + cur;
+        const float4 lx = __ldg(&w->lx), ly = __ldg(&w->ly), lz = __ldg(&w->lz), hx = __ldg(&w->hx),
+                     hy = __ldg(&w->hy), hz = __ldg(&w->hz);
+        const uint4 id = __ldg(&w->id);
+        auto push = [&](uint32_t c, float x0, float y0, float z0, float x1, float y1, float z1) {
+            float en;
+            const bool in = enters(ro, inv, x0, y0, z0, x1, y1, z1, en);
+            stack[sp] = make_uint2(c, __float_as_uint(en));  // kept if sp moves on
+            sp += (in & (en < h.t) & (c != kNone)) ? 1 : 0;
+        };
+        push(id.w, lx.w, ly.w, lz.w, hx.w, hy.w, hz.w);
+        push(id.z, lx.z, ly.z, lz.z, hx.z, hy.z, hz.z);
+        push(id.y, lx.y, ly.y, lz.y, hx.y, hy.y, hz.y);
+        push(id.x, lx.x, ly.x, lz.x, hx.x, hy.x, hz.x);
+    };
+    // Starts the ray (ro, rd).
+    auto launch = [&] {
+        h.t = 1e10f;
+        h.normal = mk(0.f, 1.f, 0.f);
+        h.tri = 0xFFFFFFFFu;
+        h.front = true;
+        inv = mk(1.0f / rd.x, 1.0f / rd.y, 1.0f / rd.z);
+        const float f = (inv.x - inv.x) + (inv.y - inv.y) + (inv.z - inv.z) + (ro.x - ro.x) +
+                        (ro.y - ro.y) + (ro.z - ro.z);
+        if (plain || f != 0.0f) {
+            trace(nodes, tris, ro, rd, h.t, h.normal, h.tri, h.front);
+            mode = kWaiting;
+        } else {
+            cur = 0;
+            sp = 0;
+            mode = kTracing;
+        }
+    };
     while (true) {
         if (!drained) {  // idle lanes take the next items
-            const unsigned need = __ballot_sync(full, !active);
+            const unsigned need = __ballot_sync(full, mode == kIdle);
             if (need) {
                 const uint32_t leader = __ffs(need) - 1;
                 uint32_t base = 0;
                 if (lane == leader) base = atomicAdd(ticket, uint32_t(__popc(need)));
                 base = __shfl_sync(full, base, leader);
                 if (base + __popc(need) >= nitems) drained = true;
-                if (!active) {
+                if (mode == kIdle) {
                     const uint32_t q = base + __popc(need & ((1u << lane) - 1u));
                     if (q < nitems) {
                         item = q;
@@ -276,19 +470,56 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_paths(RtArgs g, const NodeP* 
                         throughput = mk(1.f, 1.f, 1.f);
                         color = mk(0.f, 0.f, 0.f);
                         bounce = 0;
-                        active = true;
+                        launch();
                     }
                 }
             }
         }
-        if (__ballot_sync(full, active) == 0u) break;
-        if (!active) continue;
+        // ---- steps of the rays, until enough of them are done ----
+        const int busy = __popc(__ballot_sync(full, mode != kIdle));
+        if (busy == 0) break;
+        // the nearest entry left on the stack that is still nearer than the hit
+        auto pop = [&] {
+            cur = kNone;
+            while (sp > 0) {
+                const uint2 e = stack[--sp];
+                if (__uint_as_float(e.y) < h.t) {
+                    cur = e.x;
+                    break;
+                }
+            }
+            if (cur == kNone) mode = kWaiting;
+        };
+        while (true) {
+            const int tracing = __popc(__ballot_sync(full, mode == kTracing));
+            if (tracing == 0 || busy - tracing >= kShadeLanes) break;
+            // inner nodes, until few lanes are at one
+            while (true) {
+                const bool inner = mode == kTracing && cur < kMulti;
+                if (__popc(__ballot_sync(full, inner)) <= kInnerLanes) break;
+                if (!inner) continue;
+                visit();
+                pop();
+            }
+            if (mode == kTracing) {
+                if (cur & kLeafBit) {
+                    hit_triangle(tris, cur & ~kLeafBit, ro, rd, h);
+                } else if (cur & kMulti) {
+                    const NodeP n = nodes[cur & kNodeMask];
+                    const uint32_t lf = __float_as_uint(n.lo.w), cnt = __float_as_uint(n.hi.w) & ~kLeafBit;
+                    for (uint32_t i = 0; i < cnt; ++i) hit_triangle(tris, lf + i, ro, rd, h);
+                } else {
+                    visit();
+                }
+                pop();
+            }
+        }
+        if (mode != kWaiting) continue;
 
-        float t;
-        f3 normal;
-        uint32_t hit;
-        bool front;
-        trace(nodes, tris, ro, rd, t, normal, hit, front);
+        const float t = h.t;
+        const f3 normal = h.normal;
+        const uint32_t hit = h.tri;
+        const bool front = h.front;
         bool done = false;
         if (t >= 1e9f) {
             color = add(color, mul3(throughput, sky_color(rd)));
@@ -348,7 +579,9 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_paths(RtArgs g, const NodeP* 
         }
         if (done) {
             st3(samples, item, color);
-            active = false;
+            mode = kIdle;
+        } else {
+            launch();
         }
     }
 }
@@ -460,31 +693,44 @@ seevr_status seevr_raytrace(const seevr_rt_bindings* b, const seevr_rt_params* p
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rt_paths, kRtThreads, 0);
-    // work arrays, stream-ordered: packed nodes and triangles, per-sample
-    // colours, the path ticket
-    const size_t node_bytes = size_t(nnodes) * sizeof(NodeP), tri_bytes = size_t(p->num_triangles) * sizeof(TriP);
-    const size_t sample_bytes = size_t(nitems) * 3 * sizeof(float);
+    // work arrays, stream-ordered: wide and binary nodes, triangles, per-sample
+    // colours, parents, the path ticket
+    const size_t wide_bytes = size_t(nnodes) * sizeof(Wide), node_bytes = size_t(nnodes) * sizeof(NodeP),
+                 tri_bytes = size_t(p->num_triangles) * sizeof(TriP);
+    const size_t sample_bytes = (size_t(nitems) * 3 * sizeof(float) + 15) & ~size_t(15);
+    const size_t parent_bytes = size_t(nnodes) * sizeof(uint32_t);
+    const size_t work_bytes = wide_bytes + node_bytes + tri_bytes + sample_bytes + parent_bytes + 16;
     void* work = nullptr;
     const cudaMemPool_t pool = work_pool(dev);
-    cudaError_t e = pool ? cudaMallocFromPoolAsync(&work, node_bytes + tri_bytes + sample_bytes + 16, pool, st)
-                         : cudaMallocAsync(&work, node_bytes + tri_bytes + sample_bytes + 16, st);
+    cudaError_t e = pool ? cudaMallocFromPoolAsync(&work, work_bytes, pool, st)
+                         : cudaMallocAsync(&work, work_bytes, st);
     if (e != cudaSuccess) {
         cudaGetLastError();
         set_last_error(std::string("raytrace work arrays: ") + cudaGetErrorString(e));
         return SEEVR_ERR_OUT_OF_MEMORY;
     }
     char* w = static_cast<char*>(work);
-    NodeP* nodes = reinterpret_cast<NodeP*>(w);
-    TriP* tris = reinterpret_cast<TriP*>(w + node_bytes);
-    float* samples = reinterpret_cast<float*>(w + node_bytes + tri_bytes);
-    uint32_t* ticket = reinterpret_cast<uint32_t*>(w + node_bytes + tri_bytes + sample_bytes);
+    Wide* wide = reinterpret_cast<Wide*>(w);
+    NodeP* nodes = reinterpret_cast<NodeP*>(w + wide_bytes);
+    TriP* tris = reinterpret_cast<TriP*>(w + wide_bytes + node_bytes);
+    float* samples = reinterpret_cast<float*>(w + wide_bytes + node_bytes + tri_bytes);
+    uint32_t* parent = reinterpret_cast<uint32_t*>(w + wide_bytes + node_bytes + tri_bytes + sample_bytes);
+    uint32_t* ticket = parent + nnodes;  // and whether the tree is unfit for wide nodes
+    uint32_t* bad = ticket + 1;
     const uint32_t cap = uint32_t(std::max(sms, 1)) * 8u;
+    const uint32_t nblocks = std::min((nnodes + 255) / 256, cap);
+    cudaMemsetAsync(parent, 0xFF, parent_bytes, st);
+    // a tree of one leaf has no inner node
     cudaMemsetAsync(ticket, 0, sizeof(uint32_t), st);
-    k_rt_pack_nodes<<<std::min((nnodes + 255) / 256, cap), 256, 0, st>>>(g, nnodes, nodes);
+    cudaMemsetAsync(bad, nnodes == 1 ? 1 : 0, sizeof(uint32_t), st);
+    k_rt_pack_nodes<<<nblocks, 256, 0, st>>>(g, nnodes, nodes);
     k_rt_pack_tris<<<std::min((p->num_triangles + 255) / 256, cap), 256, 0, st>>>(g, tris);
+    k_rt_parents<<<nblocks, 256, 0, st>>>(g, nnodes, parent, bad);
+    k_rt_check<<<nblocks, 256, 0, st>>>(g, nodes, nnodes, parent, bad);
+    k_rt_wide<<<nblocks, 256, 0, st>>>(g, nodes, nnodes, bad, wide);
     const uint32_t resident = uint32_t(std::max(sms, 1)) * uint32_t(std::max(per_sm, 1));
     const uint32_t blocks = std::min((nitems + kRtThreads - 1) / kRtThreads, resident);
-    k_rt_paths<<<blocks, kRtThreads, 0, st>>>(g, nodes, tris, samples, ticket, nitems);
+    k_rt_paths<<<blocks, kRtThreads, 0, st>>>(g, nodes, wide, tris, samples, ticket, bad, nitems);
     k_rt_resolve<<<std::min(uint32_t((npix + 255) / 256), cap), 256, 0, st>>>(g, samples);
     e = cudaGetLastError();
     cudaFreeAsync(work, st);
