@@ -862,7 +862,7 @@ __global__ void __launch_bounds__(32 * W)
     if (halted(w.status)) return;  // the recomputed contacts are not valid
     const uint32_t t = threadIdx.x, lane = t & 31u, wid = t >> 5, bundle = blockIdx.x;
     const uint32_t b0 = w.bundle_off[bundle], nb = w.bundle_off[bundle + 1] - b0;
-    const uint32_t c0 = s.bundle_c0[bundle], nc = s.bundle_c0[bundle + 1] - c0;
+    const uint32_t c0 = first_contact(w, s, b0), nc = first_contact(w, s, b0 + nb) - c0;
     if (nb == 0) return;
     const bool in_smem = nb <= nbmax;
     AdjBodies B;

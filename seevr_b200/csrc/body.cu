@@ -137,6 +137,8 @@ __global__ void __launch_bounds__(kBodyThreads) k_body_stage(World w, Consts k, 
     __shared__ float sh_pose[kBodyThreads][12];  // p xyz, R by columns
     __shared__ uint32_t sh_body[kBodyThreads];
     __shared__ uint32_t sh_n;
+    start_dependents();
+    wait_for_previous();
     if (check_failed(w.status)) return;  // bounds-check mode: hull ranges not valid
     if (threadIdx.x == 0) sh_n = 0;
     __syncthreads();
@@ -281,7 +283,11 @@ int launch_body_stage(const World& w, const Consts& k, uint32_t flags, float dt,
     // render vertices in their own kernel, after the state update: the
     // per-body stage keeps its register budget (and occupancy) for the
     // substep launches
-    k_body_stage<<<blocks, kBodyThreads, 0, st>>>(w, k, flags & ~kRenderVerts, dt, gx, gy, gz, per);
+    if (flags & kIntegrate)  // after a solver's kernel
+        launch_after(k_body_stage, blocks, kBodyThreads, 0, st, w, k, flags & ~kRenderVerts, dt, gx, gy,
+                     gz, per);
+    else
+        k_body_stage<<<blocks, kBodyThreads, 0, st>>>(w, k, flags & ~kRenderVerts, dt, gx, gy, gz, per);
     if (!(flags & kRenderVerts)) return 1;
     const uint32_t rblocks = (w.nb + kRenderThreads / 32 - 1) / (kRenderThreads / 32);
     k_render_verts<<<rblocks < 148u * 64u ? rblocks : 148u * 64u, kRenderThreads, 0, st>>>(w);

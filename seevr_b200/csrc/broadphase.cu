@@ -39,6 +39,8 @@ template <bool kWrite>
 __global__ void __launch_bounds__(256) k_broad_n2(World w, const uint32_t* __restrict__ row_off,
                                                   uint32_t* __restrict__ row_count,
                                                   uint32_t* __restrict__ mask, uint32_t stride) {
+    start_dependents();
+    wait_for_previous();
     if (kWrite && halted(w.status)) return;  // row offsets from a scan that gave up
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -93,6 +95,8 @@ __global__ void __launch_bounds__(kTileThreads)
                  const uint32_t* __restrict__ row_off, uint32_t* __restrict__ row_count,
                  uint32_t* __restrict__ mask, uint32_t stride) {
     extern __shared__ float sm[];
+    start_dependents();
+    wait_for_previous();
     if (kWrite && halted(w.status)) return;  // row offsets from a scan that gave up
     uint32_t scene, slice, slices;
     if (tiles) {
@@ -225,20 +229,20 @@ int launch_broadphase_n2(const World& w, const Scratch& s, uint32_t max_scene_bo
         const uint2* tiles = s.bp_ntiles ? s.bp_tiles : nullptr;
         const uint32_t blocks = tiles ? s.bp_ntiles : w.ns * slices;
         const size_t smem = size_t(7) * max_scene_bodies * sizeof(float);
-        k_broad_tile<false><<<blocks, kTileThreads, smem, st>>>(w, tiles, slices, nullptr,
-                                                                s.row_count, s.bp_mask, s.bp_stride);
+        launch_after(k_broad_tile<false>, blocks, kTileThreads, smem, st, w, tiles, slices, nullptr,
+                     s.row_count, s.bp_mask, s.bp_stride);
         launch_exclusive_scan(s.row_count, s.row_off, nullptr, w.nb, &w.counters[0], w.max_pairs,
                               kFlagPairOverflow, s, st);
-        k_broad_tile<true><<<blocks, kTileThreads, s.bp_mask ? 0 : smem, st>>>(
-            w, tiles, slices, s.row_off, s.row_count, s.bp_mask, s.bp_stride);
+        launch_after(k_broad_tile<true>, blocks, kTileThreads, s.bp_mask ? 0 : smem, st, w, tiles, slices,
+                     s.row_off, s.row_count, s.bp_mask, s.bp_stride);
         return 3;
     }
     const uint32_t threads = 256;
     const uint32_t blocks = uint32_t((uint64_t(w.nb) * 32 + threads - 1) / threads);
-    k_broad_n2<false><<<blocks, threads, 0, st>>>(w, nullptr, s.row_count, s.bp_mask, s.bp_stride);
+    launch_after(k_broad_n2<false>, blocks, threads, 0, st, w, nullptr, s.row_count, s.bp_mask, s.bp_stride);
     launch_exclusive_scan(s.row_count, s.row_off, nullptr, w.nb, &w.counters[0], w.max_pairs,
                           kFlagPairOverflow, s, st);
-    k_broad_n2<true><<<blocks, threads, 0, st>>>(w, s.row_off, s.row_count, s.bp_mask, s.bp_stride);
+    launch_after(k_broad_n2<true>, blocks, threads, 0, st, w, s.row_off, s.row_count, s.bp_mask, s.bp_stride);
     return 3;
 }
 

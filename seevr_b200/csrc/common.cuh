@@ -134,8 +134,8 @@ struct Scratch {
     uint32_t* status;       // [4]: flags, scratch counters
     uint32_t* row_count;    // [max_bodies]   broadphase pairs per row
     uint32_t* row_off;      // [max_bodies]   exclusive scan of row_count
-    unsigned long long* scan_tiles;  // look-back tile status (+1 tile ticket)
-    uint32_t scan_tiles_cap;
+    unsigned long long* scan_tiles;  // look-back state (LookBack), zero at first
+    uint32_t scan_tiles_cap;         // its tile words
     float4* pair_res0;      // [max_pairs] contact point xyz, depth
     float4* pair_res1;      // [max_pairs] normal xyz, found flag
     uint32_t* pair_flag;    // [max_pairs] 1 if the pair makes a contact
@@ -161,7 +161,6 @@ struct Scratch {
     float* s_lam;           // [max_contacts] impulses of large bundles
     uint32_t* s_abp;        // [max_contacts*2] body pair in solve order
     float4* s_rec;          // [max_contacts*kRecWords] per-contact solver records
-    uint32_t* bundle_c0;    // [max_scenes + 1] first contact of each bundle
     // solver, per body (global-memory path for scenes too large for smem)
     float* s_R;             // [max_bodies*9]
     uint32_t* s_last;       // [max_bodies]
@@ -202,6 +201,99 @@ __device__ __forceinline__ bool halted(const uint32_t* status) {
 // since the inputs they index are not valid.
 __device__ __forceinline__ bool check_failed(const uint32_t* status) {
     return (*reinterpret_cast<const volatile uint32_t*>(status) & kFlagCheckFailed) != 0u;
+}
+
+// ---- launches that overlap the previous kernel's end --------------------------------
+// The kernels of a substep follow each other on one stream, most of them a few
+// microseconds long.  Launched with launch_after, a kernel's blocks may be set up as
+// soon as the previous kernel's have all begun (start_dependents); each waits for
+// that kernel's end, with its writes visible, before it reads anything
+// (wait_for_previous, the first thing every such kernel does).  Together with the
+// clears that LookBack saves, a frame of 25 bodies 814 -> 625 us, of 100 scenes
+// 1,567 -> 1,428 us, a large scene of 2,601 bodies 4,884 -> 3,950 us.
+__device__ __forceinline__ void start_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem,
+                                cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+// Decoupled look-back over tiles taken in ticket order.  state[0]: ticket and blocks
+// that are done; state[1]: number of the scan; then a word per tile: the scan's tag,
+// a flag (1: the tile's sum, 2: the sum up to its end) and the value.  The last block
+// of a launch resets the ticket and advances the scan's number, so that the words need
+// no clearing; when the number runs out (2^30 scans) it clears them.
+struct LookBack {
+    unsigned long long* state;
+    uint32_t tiles;  // tile words
+    uint32_t limit;  // polls of an unpublished tile
+    static constexpr uint32_t kHead = 2, kLastTag = (1u << 30) - 1u;
+    __device__ __forceinline__ uint32_t* word(uint32_t i) const {
+        return reinterpret_cast<uint32_t*>(state) + i;
+    }
+    __device__ __forceinline__ uint32_t take() const { return atomicAdd(word(0), 1u); }
+    __device__ __forceinline__ uint32_t tag() const {
+        return *reinterpret_cast<volatile uint32_t*>(word(2)) + 1u;
+    }
+    // The sum of the tiles before this one, whose own is agg.
+    __device__ __forceinline__ uint32_t before(uint32_t tile, uint32_t agg, uint32_t tag,
+                                               uint32_t* status) const {
+        unsigned long long* t = state + kHead;
+        const unsigned long long mark = static_cast<unsigned long long>(tag) << 34;
+        uint32_t excl = 0;
+        if (tile > 0) {
+            atomicExch(&t[tile], mark | (1ull << 32) | agg);
+            uint32_t spins = 0;
+            for (int p = int(tile) - 1; p >= 0;) {
+                const unsigned long long v = *reinterpret_cast<volatile unsigned long long*>(&t[p]);
+                const uint32_t f = uint32_t(v >> 34) == tag ? uint32_t(v >> 32) & 3u : 0u;
+                if (f == 0u) {
+                    if (++spins > limit) {
+                        atomicOr(status, kFlagTimeout);
+                        break;
+                    }
+                    continue;
+                }
+                excl += uint32_t(v);
+                if (f == 2u) break;
+                --p;
+            }
+        }
+        atomicExch(&t[tile], mark | (2ull << 32) | (excl + agg));
+        return excl;
+    }
+    // One thread of every block, when the block is through with the words.
+    __device__ __forceinline__ void finish() const {
+        if (atomicAdd(word(1), 1u) != gridDim.x - 1u) return;
+        const uint32_t now = *reinterpret_cast<volatile uint32_t*>(word(2)) + 1u;
+        if (now == kLastTag)
+            for (uint32_t i = 0; i < tiles; ++i) state[kHead + i] = 0ull;
+        *word(0) = 0u;
+        *word(1) = 0u;
+        *word(2) = now == kLastTag ? 0u : now;
+    }
+};
+inline LookBack look_back(const Scratch& s) { return LookBack{s.scan_tiles, s.scan_tiles_cap, s.wait_limit}; }
+
+// The first contact (of the clamped list) of bodies from `body` on: contacts follow the
+// pairs' order and pairs their rows', so it is the first contact at or after the row's
+// first pair.
+__device__ __forceinline__ uint32_t first_contact(const World& w, const Scratch& s, uint32_t body) {
+    const uint32_t total = min(w.counters[1], w.max_contacts);
+    if (body >= w.nb) return total;
+    const uint32_t p = s.row_off[body];
+    return p < min(w.counters[0], w.max_pairs) ? min(s.pair_coff[p], total) : total;
 }
 
 // ---- launchers (one translation unit each) ------------------------------
@@ -249,8 +341,6 @@ __device__ __forceinline__ uint32_t lut_of(const World& w, uint32_t b) {
 int launch_narrowphase_taped(const World& w, const Consts& k, const Scratch& s, uint4* pair_tape,
                              uint4* contact_tape, cudaStream_t st);
 cudaError_t init_solver();
-// bundle_c0: the first contact of every solver bundle (one marking pass)
-int launch_bundle_ranges(const World& w, const Scratch& s, cudaStream_t st);
 // Set the calling thread's message returned by seevr_last_error().
 void set_last_error(const char* msg);
 inline void set_last_error(const std::string& msg) { set_last_error(msg.c_str()); }

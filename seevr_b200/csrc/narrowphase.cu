@@ -455,6 +455,8 @@ __global__ void __launch_bounds__(kNarrowThreads, kMinBlocks)
              const uint32_t* __restrict__ order) {
     __shared__ float wit[4][Witness<kTape>::kWords][kNarrowThreadsW];
     __shared__ float pose[2][12][kNarrowThreadsW];
+    start_dependents();
+    wait_for_previous();
     if (halted(w.status)) return;  // pairs from a scan that gave up
     const uint32_t np = min(w.counters[0], w.max_pairs);
     const uint32_t lane = threadIdx.x & 31u;
@@ -904,7 +906,10 @@ __global__ void k_contact_scatter(World w, const float4* __restrict__ res0,
                                   const uint32_t* __restrict__ flag,
                                   const uint32_t* __restrict__ coff,
                                   const uint4* __restrict__ pair_tape,
-                                  uint4* __restrict__ contact_tape) {
+                                  uint4* __restrict__ contact_tape, uint32_t* ticket) {
+    start_dependents();
+    wait_for_previous();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0u;  // the narrowphase's
     if (halted(w.status)) return;  // offsets from a scan that gave up
     const uint32_t np = min(w.counters[0], w.max_pairs);
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
@@ -929,8 +934,7 @@ int launch_narrowphase_taped(const World& w, const Consts& k, const Scratch& s, 
                              uint4* contact_tape, cudaStream_t st) {
     if (w.max_pairs == 0) return 0;
     // persistent grid: a few resident blocks per SM; the pair ticket lives
-    // in status[1] and is cleared here
-    cudaMemsetAsync(&s.status[1], 0, sizeof(uint32_t), st);
+    // in status[1], zero between launches (k_contact_scatter clears it)
     // (four lanes per pair that the buffers can hold, so that few pairs get
     // sixteen each)
     const uint32_t most = s.narrow_blocks ? s.narrow_blocks : 148 * kNarrowBlocksPerSm;
@@ -955,16 +959,16 @@ int launch_narrowphase_taped(const World& w, const Consts& k, const Scratch& s, 
     } else {
         const Out o{s.pair_res0, s.pair_res1, s.pair_flag, pair_tape};
         uint32_t* ticket = &s.status[1];
-        if (pair_tape && seven) k_narrow<true, 7><<<blocks, kNarrowThreads, 0, st>>>(w, k, o, ticket, order);
-        else if (pair_tape) k_narrow<true, 6><<<blocks, kNarrowThreads, 0, st>>>(w, k, o, ticket, order);
-        else if (seven) k_narrow<false, 7><<<blocks, kNarrowThreads, 0, st>>>(w, k, o, ticket, order);
-        else k_narrow<false, 6><<<blocks, kNarrowThreads, 0, st>>>(w, k, o, ticket, order);
+        if (pair_tape && seven) launch_after(k_narrow<true, 7>, blocks, kNarrowThreads, 0, st, w, k, o, ticket, order);
+        else if (pair_tape) launch_after(k_narrow<true, 6>, blocks, kNarrowThreads, 0, st, w, k, o, ticket, order);
+        else if (seven) launch_after(k_narrow<false, 7>, blocks, kNarrowThreads, 0, st, w, k, o, ticket, order);
+        else launch_after(k_narrow<false, 6>, blocks, kNarrowThreads, 0, st, w, k, o, ticket, order);
     }
     launch_exclusive_scan(s.pair_flag, s.pair_coff, &w.counters[0], w.max_pairs,
                           &w.counters[1], w.max_contacts, kFlagContactOverflow, s, st);
-    k_contact_scatter<<<grid_for(w.max_pairs, 256, 148 * 16), 256, 0, st>>>(
-        w, s.pair_res0, s.pair_res1, s.pair_flag, s.pair_coff, pair_tape,
-        pair_tape ? contact_tape : nullptr);
+    launch_after(k_contact_scatter, grid_for(w.max_pairs, 256, 148 * 16), 256, 0, st, w, s.pair_res0,
+                 s.pair_res1, s.pair_flag, s.pair_coff, pair_tape, pair_tape ? contact_tape : nullptr,
+                 &s.status[1]);
     return n;
 }
 

@@ -10,12 +10,12 @@
 // entry point runs the same kernels on scratch carved from one file-scope
 // device array, so the caller provides only the bound buffers and a stream.
 //
-// The array holds SEEVR_NOALLOC_SCRATCH_BYTES (5,489,920 bytes, about 5.5 MB)
-// on every device that loads the library, until the process exits.  All calls share it: calls whose GPU
-// work overlaps (different streams, or different host threads on one
-// device) race on it and must be serialised by the caller.  Each call
-// clears the parts that must start at zero (the status word, scan and
-// solver state are reset by the kernels themselves).
+// The array holds SEEVR_NOALLOC_SCRATCH_BYTES (5,489,664 bytes, about 5.5 MB)
+// on every device that loads the library, until the process exits.  All
+// calls share it: calls whose GPU work overlaps (different streams, or
+// different host threads on one device) race on it and must be serialised by
+// the caller.  Each call clears the parts that must start at zero (the status
+// words and the scans' look-back state; the kernels reset the rest).
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -30,7 +30,7 @@ namespace {
 constexpr uint32_t kNaBodies = SEEVR_NOALLOC_MAX_BODIES;
 constexpr uint32_t kNaPairs = SEEVR_NOALLOC_MAX_PAIRS;
 constexpr uint32_t kNaContacts = SEEVR_NOALLOC_MAX_CONTACTS;
-constexpr uint32_t kNaScanTiles = (kNaPairs > kNaBodies ? kNaPairs : kNaBodies) / 2048 + 2;
+constexpr uint32_t kNaScanTiles = (kNaPairs > kNaBodies ? kNaPairs : kNaBodies) / 2048 + 1;
 
 // Byte layout of the scratch array (each region 256-byte aligned).
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -38,7 +38,7 @@ constexpr size_t kOffStatus = 0;
 constexpr size_t kOffRowCount = align256(kOffStatus + 16);
 constexpr size_t kOffRowOff = align256(kOffRowCount + 4ull * kNaBodies);
 constexpr size_t kOffScanTiles = align256(kOffRowOff + 4ull * kNaBodies);
-constexpr size_t kOffRes0 = align256(kOffScanTiles + 8ull * kNaScanTiles);
+constexpr size_t kOffRes0 = align256(kOffScanTiles + 8ull * (kNaScanTiles + LookBack::kHead));
 constexpr size_t kOffRes1 = align256(kOffRes0 + 16ull * kNaPairs);
 constexpr size_t kOffFlag = align256(kOffRes1 + 16ull * kNaPairs);
 constexpr size_t kOffCoff = align256(kOffFlag + 4ull * kNaPairs);
@@ -59,8 +59,7 @@ constexpr size_t kOffSceneOff = align256(kOffBodyScene + 4ull * kNaBodies);
 constexpr size_t kOffN = align256(kOffSceneOff + 8);
 constexpr size_t kOffLam = align256(kOffN + 12ull * kNaContacts);
 constexpr size_t kOffAbp = align256(kOffLam + 4ull * kNaContacts);
-constexpr size_t kOffBundleC0 = align256(kOffAbp + 8ull * kNaContacts);
-constexpr size_t kOffRec = align256(kOffBundleC0 + 16);
+constexpr size_t kOffRec = align256(kOffAbp + 8ull * kNaContacts);
 constexpr size_t kNaBytes = align256(kOffRec + 16ull * kRecWords * kNaContacts);
 static_assert(kNaBytes == SEEVR_NOALLOC_SCRATCH_BYTES, "header constant out of date");
 
@@ -208,7 +207,6 @@ extern "C" seevr_status seevr_physics_step_noalloc(
     s.s_n = reinterpret_cast<float*>(at(kOffN));
     s.s_lam = reinterpret_cast<float*>(at(kOffLam));
     s.s_abp = reinterpret_cast<uint32_t*>(at(kOffAbp));
-    s.bundle_c0 = reinterpret_cast<uint32_t*>(at(kOffBundleC0));
     s.s_rec = reinterpret_cast<float4*>(at(kOffRec));
     uint32_t* body_scene = reinterpret_cast<uint32_t*>(at(kOffBodyScene));
     uint32_t* scene_off = reinterpret_cast<uint32_t*>(at(kOffSceneOff));
@@ -270,9 +268,10 @@ extern "C" seevr_status seevr_physics_step_noalloc(
     k.narrowphase = p.narrowphase <= SEEVR_NARROWPHASE_GJK_EPA ? p.narrowphase : 0u;
 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // state the kernels expect to start from: a clear status word, the one
-    // scene's body map and (without binding 30) the hull ranges
+    // state the kernels expect to start from: a clear status word and look-back
+    // state, the one scene's body map and (without binding 30) the hull ranges
     cudaMemsetAsync(s.status, 0, 16, st);
+    cudaMemsetAsync(s.scan_tiles, 0, 8ull * (kNaScanTiles + LookBack::kHead), st);
     k_noalloc_one_scene<<<(num_bodies + 255) / 256, 256, 0, st>>>(body_scene, scene_off, num_bodies);
     if (!ext_range)
         launch_hull_range_from_geom_data(static_cast<const float*>(P(SEEVR_B_GEOM_DATA)),

@@ -866,7 +866,7 @@ seevr_status seevr_physics_create(const seevr_bindings* b, const seevr_caps* cap
     seevr_status st = SEEVR_OK;
     const seevr_caps& c = h->caps;
     const uint32_t scan_n = std::max(std::max(std::max(c.max_bodies, c.max_pairs), c.max_contacts), 1u);
-    h->s.scan_tiles_cap = (scan_n + 2047) / 2048 + 2;
+    h->s.scan_tiles_cap = (scan_n + 2047) / 2048 + 1;
     h->s.wait_limit = kSpinLimit;
     h->lb.wait_limit = kSpinLimit;
     if (const char* e = std::getenv("SEEVR_CHECK")) h->check = std::strcmp(e, "1") == 0;
@@ -875,7 +875,7 @@ seevr_status seevr_physics_create(const seevr_bindings* b, const seevr_caps* cap
     ALLOC(h->s.status, 4);
     ALLOC(h->s.row_count, c.max_bodies);
     ALLOC(h->s.row_off, c.max_bodies);
-    ALLOC(h->s.scan_tiles, h->s.scan_tiles_cap);
+    ALLOC(h->s.scan_tiles, h->s.scan_tiles_cap + LookBack::kHead);
     ALLOC(h->s.pair_res0, c.max_pairs);
     ALLOC(h->s.pair_res1, c.max_pairs);
     ALLOC(h->s.pair_flag, c.max_pairs);
@@ -896,7 +896,6 @@ seevr_status seevr_physics_create(const seevr_bindings* b, const seevr_caps* cap
     ALLOC(h->s.s_lam, c.max_contacts);
     ALLOC(h->s.s_abp, size_t(c.max_contacts) * 2);
     ALLOC(h->s.s_rec, size_t(c.max_contacts) * kRecWords);
-    ALLOC(h->s.bundle_c0, size_t(c.max_scenes) + 2);
     ALLOC(h->body_bundle, c.max_bodies);
     ALLOC(h->s.s_R, size_t(c.max_bodies) * 9);
     ALLOC(h->s.s_last, c.max_bodies);
@@ -964,7 +963,9 @@ seevr_status seevr_physics_create(const seevr_bindings* b, const seevr_caps* cap
     if (st == SEEVR_OK && (cudaEventCreate(&h->ev[0]) != cudaSuccess ||
                            cudaEventCreate(&h->ev[1]) != cudaSuccess))
         st = fail(SEEVR_ERR_CUDA, "cudaEventCreate failed");
-    if (st == SEEVR_OK && cudaMemset(h->s.status, 0, 16) != cudaSuccess)
+    if (st == SEEVR_OK &&
+        (cudaMemset(h->s.status, 0, 16) != cudaSuccess ||
+         cudaMemset(h->s.scan_tiles, 0, 8 * size_t(h->s.scan_tiles_cap + LookBack::kHead)) != cudaSuccess))
         st = fail(SEEVR_ERR_CUDA, "cudaMemset failed");
     if (st == SEEVR_OK && init_solver() != cudaSuccess)
         st = fail(SEEVR_ERR_CUDA, "cudaFuncSetAttribute for the solver failed");
@@ -1380,7 +1381,6 @@ seevr_status seevr_physics_adjoint_substep(seevr_physics* h, uint32_t num_bodies
                                                        : launch_broadphase_n2(w, h->s, h->max_scene_bodies, s);
     n += launch_lut_alias(w, h->s, s);
     n += launch_narrowphase_taped(w, h->k, h->s, a.ptape, a.ctape, s);
-    n += launch_bundle_ranges(w, h->s, s);
     const Grads g{grads->pos, grads->quat, grads->vel, grads->omega, grads->friction};
     n += launch_adjoint(w, h->k, h->s, a, g, dt, h->max_bundle_bodies, s);
     h->launches += n;

@@ -8,7 +8,8 @@
 // wait limit, kSpinLimit polls by default) and raises kFlagTimeout instead
 // of hanging.  Offsets written after a wait gave up are too small but stay
 // within `out`; the kernels that would use them see the timeout bit and
-// return (timed_out).
+// return (timed_out).  The look-back words carry the number of the scan that
+// wrote them (LookBack, common.cuh), so no launch clears them beforehand.
 #include "common.cuh"
 
 namespace seevr {
@@ -17,23 +18,27 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;  // 2048
 
-__device__ __forceinline__ unsigned long long ld_volatile(const unsigned long long* p) {
-    return *reinterpret_cast<const volatile unsigned long long*>(p);
-}
-
 __global__ void __launch_bounds__(kScanThreads)
     k_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, const uint32_t* n_dev,
            uint32_t n_cap, uint32_t* total_out, uint32_t total_cap, uint32_t overflow_bit,
-           unsigned long long* tiles, uint32_t* status, uint32_t wait_limit) {
-    __shared__ uint32_t s_tile, s_excl;
+           LookBack lb, uint32_t* status) {
+    __shared__ uint32_t s_tile, s_excl, s_tag;
     __shared__ uint32_t s_warp[kScanThreads / 32];
+    start_dependents();
+    wait_for_previous();
     const uint32_t n = n_dev ? min(*n_dev, n_cap) : n_cap;
     const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;
-    if (threadIdx.x == 0) s_tile = atomicAdd(reinterpret_cast<unsigned int*>(tiles), 1u);
+    if (threadIdx.x == 0) {
+        s_tile = lb.take();
+        s_tag = lb.tag();
+    }
     __syncthreads();
     const uint32_t tile = s_tile;
     if (tile >= ntiles) {
-        if (n == 0 && tile == 0 && threadIdx.x == 0 && total_out) *total_out = 0;
+        if (threadIdx.x == 0) {
+            if (n == 0 && tile == 0 && total_out) *total_out = 0;
+            lb.finish();
+        }
         return;
     }
     const uint32_t base = tile * kScanTile + threadIdx.x * kScanItems;
@@ -66,36 +71,14 @@ __global__ void __launch_bounds__(kScanThreads)
         if (lane == kScanThreads / 32 - 1) {
             // lane 7 holds the block aggregate in wi; look back
             const uint32_t agg = wi;
-            unsigned long long* st = tiles + 1;
-            uint32_t excl = 0;
-            if (tile == 0) {
-                atomicExch(&st[0], (2ull << 32) | agg);
-            } else {
-                atomicExch(&st[tile], (1ull << 32) | agg);
-                int p = int(tile) - 1;
-                uint32_t spins = 0;
-                while (p >= 0) {
-                    const unsigned long long s = ld_volatile(&st[p]);
-                    const uint32_t f = uint32_t(s >> 32);
-                    if (f == 0u) {
-                        if (++spins > wait_limit) {
-                            atomicOr(status, kFlagTimeout);
-                            break;
-                        }
-                        continue;
-                    }
-                    excl += uint32_t(s);
-                    if (f == 2u) break;
-                    --p;
-                }
-                atomicExch(&st[tile], (2ull << 32) | (excl + agg));
-            }
+            const uint32_t excl = lb.before(tile, agg, s_tag, status);
             s_excl = excl;
             if (tile == ntiles - 1) {
                 const uint32_t total = excl + agg;
                 if (total_out) *total_out = total;
                 if (total > total_cap) atomicOr(status, overflow_bit);
             }
+            lb.finish();
         }
     }
     __syncthreads();
@@ -111,10 +94,8 @@ int launch_exclusive_scan(const uint32_t* in, uint32_t* out, const uint32_t* n_d
                           uint32_t n_cap, uint32_t* total_out, uint32_t total_cap,
                           uint32_t overflow_bit, const Scratch& s, cudaStream_t st) {
     const uint32_t tiles = (n_cap + kScanTile - 1) / kScanTile;
-    const uint32_t blocks = tiles > 0 ? tiles : 1;
-    cudaMemsetAsync(s.scan_tiles, 0, sizeof(unsigned long long) * (blocks + 1), st);
-    k_scan<<<blocks, kScanThreads, 0, st>>>(in, out, n_dev, n_cap, total_out, total_cap,
-                                            overflow_bit, s.scan_tiles, s.status, s.wait_limit);
+    launch_after(k_scan, tiles > 0 ? tiles : 1, kScanThreads, 0, st, in, out, n_dev, n_cap,
+                 total_out, total_cap, overflow_bit, look_back(s), s.status);
     return 1;
 }
 

@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(kSolverThreads)
     const uint32_t scene = blockIdx.x;  // bundle index
     const uint32_t b0 = w.bundle_off[scene], b1 = w.bundle_off[scene + 1];
     const uint32_t nbs = b1 - b0;
-    const uint32_t c0 = s.bundle_c0[scene], c1 = s.bundle_c0[scene + 1];
+    const uint32_t c0 = first_contact(w, s, b0), c1 = first_contact(w, s, b1);
     if (c0 >= c1) return;
     const uint32_t tid = threadIdx.x;
 
@@ -179,21 +179,6 @@ __global__ void __launch_bounds__(kSolverThreads)
             st3(w.vel, b0 + i, ld3(B.v, i));
             st3(w.omega, b0 + i, ld3(B.w, i));
         }
-    }
-}
-
-// ---- contact range of every bundle ----------------------------------------
-// Contacts are in (a, b) order and bundles own consecutive body ranges, so
-// each bundle's contacts form one run; bundle_c0[k] = first contact of bundle
-// k (bundle_c0[nbundles] = the contact count).  Marked in one pass instead of
-// a binary search at the start of every solver block.
-__global__ void k_bundle_ranges(World w, uint32_t* __restrict__ bundle_c0) {
-    if (halted(w.status)) return;  // contacts from a scan that gave up
-    const uint32_t nc = min(w.counters[1], w.max_contacts);
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= nc; c += gridDim.x * blockDim.x) {
-        const uint32_t cur = c < nc ? w.body_bundle[w.geom_body[w.c_a[c]]] : w.nbundles;
-        const int prev = c > 0 ? int(w.body_bundle[w.geom_body[w.c_a[c - 1]]]) : -1;
-        for (int k = prev + 1; k <= int(cur); ++k) bundle_c0[k] = c;
     }
 }
 
@@ -552,12 +537,14 @@ __global__ void __launch_bounds__(32 * W, 12 / W)
     constexpr uint32_t kThreads = 32 * W;
     extern __shared__ float4 sm4[];
     __shared__ uint32_t sh_order, sh_left, sh_chained, sh_ticket;
+    start_dependents();
+    wait_for_previous();
     if (halted(w.status)) return;  // contacts from a scan that gave up
     const uint32_t t = threadIdx.x, lane = t & 31u, wid = t >> 5;
     const uint32_t bundle = blockIdx.x;
     if (bundle >= w.nbundles) return;
-    const uint32_t c0 = s.bundle_c0[bundle], c1 = s.bundle_c0[bundle + 1];
     const uint32_t b0 = w.bundle_off[bundle], b1 = w.bundle_off[bundle + 1];
+    const uint32_t c0 = first_contact(w, s, b0), c1 = first_contact(w, s, b1);
     if (c0 >= c1) return;
     const uint32_t nbs = b1 - b0, nc = c1 - c0;
     const FlowBodies B{sm4, sm4 + nbmax};
@@ -693,13 +680,6 @@ cudaError_t init_solver() {
                                 int(kSolverMaxSmem));
 }
 
-int launch_bundle_ranges(const World& w, const Scratch& s, cudaStream_t st) {
-    uint32_t rb = (w.max_contacts + 1 + 255) / 256;
-    if (rb > 148u * 8u) rb = 148u * 8u;
-    k_bundle_ranges<<<rb, 256, 0, st>>>(w, s.bundle_c0);
-    return 1;
-}
-
 // Warps per block by the largest bundle: a settled pile has about a quarter
 // contact per body, two thirds of them chained, and the warps without chained
 // contacts take the lone ones.  Solver time per substep with 1 / 2 / 4 warps:
@@ -716,28 +696,27 @@ static void launch_flow(const World& w, const Consts& k, const Scratch& s, uint3
     const uint32_t recs = budget > base ? (budget - base) / (16 * kRecWords) : 0u;
     const uint32_t smem = flow_smem_bytes(nbmax, recs);
     switch (warps) {
-        case 1: k_solver_flow<1><<<w.nbundles, 32, smem, st>>>(w, k, s, mode, dt, nbmax, recs); break;
-        case 2: k_solver_flow<2><<<w.nbundles, 64, smem, st>>>(w, k, s, mode, dt, nbmax, recs); break;
-        case 4: k_solver_flow<4><<<w.nbundles, 128, smem, st>>>(w, k, s, mode, dt, nbmax, recs); break;
-        default: k_solver_flow<8><<<w.nbundles, 256, smem, st>>>(w, k, s, mode, dt, nbmax, recs);
+        case 1: launch_after(k_solver_flow<1>, w.nbundles, 32, smem, st, w, k, s, mode, dt, nbmax, recs); break;
+        case 2: launch_after(k_solver_flow<2>, w.nbundles, 64, smem, st, w, k, s, mode, dt, nbmax, recs); break;
+        case 4: launch_after(k_solver_flow<4>, w.nbundles, 128, smem, st, w, k, s, mode, dt, nbmax, recs); break;
+        default: launch_after(k_solver_flow<8>, w.nbundles, 256, smem, st, w, k, s, mode, dt, nbmax, recs);
     }
 }
 
 int launch_solver(const World& w, const Consts& k, const Scratch& s, uint32_t mode, float dt,
                   uint32_t max_scene_bodies, cudaStream_t st) {
     if (w.nbundles == 0 || w.max_contacts == 0) return 0;
-    launch_bundle_ranges(w, s, st);
     if (max_scene_bodies <= kWarpMaxBodies) {
         launch_flow(w, k, s, mode, dt, std::max(max_scene_bodies, 1u), st);
-        return 2;
+        return 1;
     }
-    if (s.isl.parent) return 1 + launch_solver_islands(w, k, s, mode, dt, st);
+    if (s.isl.parent) return launch_solver_islands(w, k, s, mode, dt, st);
     uint32_t cta_bodies = max_scene_bodies;
     if (cta_bodies * kBodySmemWords * 4 > kSolverMaxSmem)
         cta_bodies = kSolverMaxSmem / (kBodySmemWords * 4);
     const size_t smem = size_t(cta_bodies) * kBodySmemWords * 4;
     k_solver<<<w.nbundles, kSolverThreads, smem, st>>>(w, k, s, mode, dt, cta_bodies);
-    return 2;
+    return 1;
 }
 
 }  // namespace seevr
