@@ -122,7 +122,7 @@ struct IslandScratch {
     uint32_t* head;         // [max_contacts] 1 at an island's first slot
     uint32_t* idx;          // [max_contacts] exclusive scan of head
     uint32_t* start;        // [max_contacts + 1] first slot of each island
-    uint32_t* count;        // [1] islands
+    uint32_t* count;        // [3] islands; the run kernel's ticket; islands left over
     uint32_t* lvl;          // [2 * max_contacts + 2] level boundaries per island
     uint32_t* sort_hist;    // [4 * 256]
     uint32_t* sort_status;  // look-back words of the sort
@@ -349,6 +349,11 @@ int launch_solver(const World& w, const Consts& k, const Scratch& s, uint32_t mo
                   float dt, uint32_t max_scene_bodies, cudaStream_t st);
 // Island-parallel solve of the whole contact list (needs s.isl); mode 0
 // sequential, 1 wavefront, 2 coloured.
+// Islands of at most kIslandMost contacts, in runs (solver.cu); todo[i]: 1 for the
+// islands that are left over.
+constexpr uint32_t kIslandMost = 1024;
+int launch_island_flow(const World& w, const Consts& k, const Scratch& s, uint32_t mode, float dt,
+                       uint32_t sms, uint32_t* todo, uint32_t* left, cudaStream_t st);
 int launch_solver_islands(const World& w, const Consts& k, const Scratch& s, uint32_t mode,
                           float dt, cudaStream_t st);
 // Grid-wide coloured solve of the islands above kGiantContacts contacts (a

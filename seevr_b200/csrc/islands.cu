@@ -9,16 +9,22 @@
 // island replaces one block per scene.
 //
 // Per substep:
-//   1. union-find over the dynamic bodies of every contact (lock-free
-//      hooking of the larger root under the smaller, so the final root of a
-//      component is its smallest body index, whatever the schedule);
+//   1. union-find over the dynamic bodies of every contact: each body is linked
+//      to its smallest smaller partner, the links are shortened by all bodies
+//      at once (a tower of 256 boxes is a path of 255 links, which one thread
+//      walking it takes 80 us for), and the remaining contacts are joined by
+//      lock-free hooking of the larger root under the smaller, so the final
+//      root of a component is its smallest body index, whatever the schedule;
 //   2. key = island root per contact (skipped contacts sort last), and a
 //      stable radix sort of (key, contact), which keeps each island's
 //      contacts in index order;
 //   3. island starts from the key changes (one exclusive scan);
-//   4. a persistent grid of warps takes islands in turn: levels (WAVEFRONT),
-//      greedy colours (COLORED) or one level (SEQUENTIAL), then the sweep
-//      with the body state in place in global memory.
+//   4. runs of whole islands are solved by a block each, in dataflow order
+//      (k_island_flow, solver.cu), except in mode SEQUENTIAL;
+//   5. a persistent grid of warps takes the islands that are left over in turn:
+//      levels (WAVEFRONT), greedy colours (COLORED) or one level
+//      (SEQUENTIAL), then the sweep with the body state in place in global
+//      memory.
 #include "common.cuh"
 #include "lbvh.cuh"
 #include "solver.cuh"
@@ -54,7 +60,10 @@ __device__ __forceinline__ uint32_t find_root(uint32_t* parent, uint32_t x) {
 // Every island kernel runs on contacts from the narrowphase's scan (and the
 // later ones on the island sort): none runs after a wait gave up.
 __global__ void k_island_prep(World w, Scratch s) {
+    start_dependents();
+    wait_for_previous();
     if (halted(w.status)) return;
+    if (blockIdx.x == 0 && threadIdx.x < 3) s.isl.count[threadIdx.x] = 0;
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < w.nb; b += gridDim.x * blockDim.x) {
         s.isl.parent[b] = b;
         s.s_last[b] = 0;
@@ -62,15 +71,51 @@ __global__ void k_island_prep(World w, Scratch s) {
     }
 }
 
-// Hook the roots of a contact's two dynamic bodies: a failed CAS returns a
-// smaller root, so every retry makes progress.
-__global__ void k_island_union(World w, Scratch s) {
+// Both bodies of a contact, if it joins their islands.
+__device__ __forceinline__ bool joins(const World& w, uint32_t c, uint32_t& a, uint32_t& b) {
+    a = w.geom_body[w.c_a[c]];
+    b = w.geom_body[w.c_b[c]];
+    if (w.inv_mass[a] == 0.0f && w.inv_mass[b] == 0.0f) return false;  // skipped (physics.comp:531)
+    return !body_fixed(w, a) && !body_fixed(w, b);
+}
+
+__global__ void k_island_link(World w, Scratch s) {
+    start_dependents();
+    wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t nc = min(w.counters[1], w.max_contacts);
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-        const uint32_t a = w.geom_body[w.c_a[c]], b = w.geom_body[w.c_b[c]];
-        if (w.inv_mass[a] == 0.0f && w.inv_mass[b] == 0.0f) continue;  // skipped (physics.comp:531)
-        if (body_fixed(w, a) || body_fixed(w, b)) continue;
+        uint32_t a, b;
+        if (joins(w, c, a, b)) atomicMin(&s.isl.parent[max(a, b)], min(a, b));
+    }
+}
+
+// Every body's link to its root.  A body takes over its parent's link, while that
+// body does the same, so the links' lengths double; each step goes to a smaller index.
+__global__ void k_island_shorten(World w, Scratch s) {
+    start_dependents();
+    wait_for_previous();
+    if (halted(w.status)) return;
+    volatile uint32_t* p = s.isl.parent;
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < w.nb; b += gridDim.x * blockDim.x) {
+        uint32_t cur = p[b], next;
+        while ((next = p[cur]) < cur) {
+            p[b] = next;
+            cur = next;
+        }
+    }
+}
+
+// Hook the roots of a contact's two dynamic bodies: a failed CAS returns a
+// smaller root, so every retry makes progress.
+__global__ void k_island_union(World w, Scratch s) {
+    start_dependents();
+    wait_for_previous();
+    if (halted(w.status)) return;
+    const uint32_t nc = min(w.counters[1], w.max_contacts);
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
+        uint32_t a, b;
+        if (!joins(w, c, a, b)) continue;
         uint32_t ra = find_root(s.isl.parent, a), rb = find_root(s.isl.parent, b);
         while (ra != rb) {
             if (ra > rb) {
@@ -86,6 +131,8 @@ __global__ void k_island_union(World w, Scratch s) {
 }
 
 __global__ void k_island_keys(World w, Scratch s) {
+    start_dependents();
+    wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t nc = min(w.counters[1], w.max_contacts);
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < w.max_contacts;
@@ -102,6 +149,8 @@ __global__ void k_island_keys(World w, Scratch s) {
 }
 
 __global__ void k_island_heads(World w, Scratch s) {
+    start_dependents();
+    wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t* k = s.isl.keys_out;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < w.max_contacts;
@@ -110,6 +159,8 @@ __global__ void k_island_heads(World w, Scratch s) {
 }
 
 __global__ void k_island_starts(World w, Scratch s) {
+    start_dependents();
+    wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t* k = s.isl.keys_out;
     const uint32_t n = w.max_contacts;
@@ -124,8 +175,12 @@ __global__ void k_island_starts(World w, Scratch s) {
 // Warp per island (persistent).  Positions p in [start, start+1) index the
 // island's contacts in index order (perm[p] = contact).
 __global__ void __launch_bounds__(kIslandThreads)
-    k_solver_island(World w, Consts k, Scratch s, uint32_t mode, float dt, uint32_t giant) {
+    k_solver_island(World w, Consts k, Scratch s, uint32_t mode, float dt, uint32_t giant,
+                    const uint32_t* __restrict__ todo) {
+    start_dependents();
+    wait_for_previous();
     if (halted(w.status)) return;
+    if (todo && s.isl.count[2] == 0) return;
     const unsigned full = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -135,7 +190,8 @@ __global__ void __launch_bounds__(kIslandThreads)
     uint32_t* last = s.s_last;
     for (uint32_t isl = gwarp; isl < count; isl += nwarps) {
         const uint32_t p0 = s.isl.start[isl], p1 = s.isl.start[isl + 1];
-        if (p1 - p0 > giant) continue;  // solved grid-wide (giant.cu)
+        if (p1 - p0 > giant) continue;    // solved grid-wide (giant.cu)
+        if (todo && !todo[isl]) continue;  // solved in a run (k_island_flow)
         for (uint32_t i = p0 + lane; i < p1; i += 32) {
             const uint32_t c = perm[i];
             s.s_ab[size_t(i) * 2] = w.geom_body[w.c_a[c]];
@@ -287,19 +343,21 @@ int launch_solver_islands(const World& w, const Consts& k, const Scratch& s, uin
     if (w.max_contacts == 0) return 0;
     const uint32_t cap = 148u * 8u;
     const uint32_t nbb = min(blocks_of(w.nb, 256), cap), ncb = min(blocks_of(w.max_contacts, 256), cap);
-    k_island_prep<<<nbb, 256, 0, st>>>(w, s);
-    k_island_union<<<ncb, 256, 0, st>>>(w, s);
-    k_island_keys<<<ncb, 256, 0, st>>>(w, s);
+    launch_after(k_island_prep, nbb, 256, 0, st, w, s);
+    launch_after(k_island_link, ncb, 256, 0, st, w, s);
+    launch_after(k_island_shorten, nbb, 256, 0, st, w, s);
+    launch_after(k_island_union, ncb, 256, 0, st, w, s);
+    launch_after(k_island_keys, ncb, 256, 0, st, w, s);
     LbvhScratch ls{};
     ls.hist = s.isl.sort_hist;
     ls.status = s.isl.sort_status;
     ls.wait_limit = s.wait_limit;
-    int n = 3 + lbvh_sort(s.isl.keys_in, s.isl.vals_in, s.isl.keys_tmp, s.isl.vals_tmp,
+    int n = 5 + lbvh_sort(s.isl.keys_in, s.isl.vals_in, s.isl.keys_tmp, s.isl.vals_tmp,
                           s.isl.keys_out, s.isl.perm, w.max_contacts, ls, &s.status[0], st);
-    k_island_heads<<<ncb, 256, 0, st>>>(w, s);
+    launch_after(k_island_heads, ncb, 256, 0, st, w, s);
     n += 1 + launch_exclusive_scan(s.isl.head, s.isl.idx, nullptr, w.max_contacts, s.isl.count,
                                    w.max_contacts + 1, 0u, s, st);
-    k_island_starts<<<ncb, 256, 0, st>>>(w, s);
+    launch_after(k_island_starts, ncb, 256, 0, st, w, s);
     static int per_sm = 0;
     if (per_sm == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solver_island, kIslandThreads, 0);
@@ -311,8 +369,12 @@ int launch_solver_islands(const World& w, const Consts& k, const Scratch& s, uin
     // coloured mode: islands above kGiantContacts contacts are solved by the
     // whole grid, the others by a warp each
     const int giant = mode == 2 ? launch_solver_giant(w, k, s, dt, st) : 0;
-    k_solver_island<<<uint32_t(sms) * uint32_t(per_sm), kIslandThreads, 0, st>>>(
-        w, k, s, mode, dt, giant ? (s.giant_min ? s.giant_min : kGiantContacts) : 0xFFFFFFFFu);
+    const uint32_t giant_min = giant ? (s.giant_min ? s.giant_min : kGiantContacts) : 0xFFFFFFFFu;
+    // (keys_tmp: free after the sort)
+    uint32_t* todo = mode != 0 && giant_min > kIslandMost ? s.isl.keys_tmp : nullptr;
+    if (todo) n += launch_island_flow(w, k, s, mode, dt, uint32_t(sms), todo, s.isl.count + 1, st);
+    launch_after(k_solver_island, uint32_t(sms) * uint32_t(per_sm), kIslandThreads, 0, st, w, k, s, mode,
+                 dt, giant_min, static_cast<const uint32_t*>(todo));
     return n + 2 + giant;
 }
 

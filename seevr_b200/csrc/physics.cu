@@ -916,7 +916,7 @@ seevr_status seevr_physics_create(const seevr_bindings* b, const seevr_caps* cap
         ALLOC(is.head, nc);
         ALLOC(is.idx, nc);
         ALLOC(is.start, nc + 1);
-        ALLOC(is.count, 1);
+        ALLOC(is.count, 3);
         ALLOC(is.lvl, 2 * nc + 2);
         ALLOC(is.sort_hist, 4 * 256);
         ALLOC(is.sort_status, lbvh_status_words(c.max_contacts));

@@ -285,9 +285,12 @@ __device__ __forceinline__ bool colour_sides(uint32_t* info, const FlowBodies& B
     const unsigned full = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t ok = 1u, mx = 0u;
-    if (lane == 0)
+    if (lane == 0) {
+        const uint2* sides = reinterpret_cast<const uint2*>(info);
+        uint2 next = sides[0];
         for (uint32_t i = 0; i < nc && ok; ++i) {
-            const uint32_t a = info[2 * i], b = info[2 * i + 1];
+            const uint32_t a = next.x, b = next.y;
+            if (i + 1 < nc) next = sides[i + 1];
             if (a & kSideSkip) {
                 level[i] = 0u;  // solved by nobody: any colour
                 continue;
@@ -301,6 +304,7 @@ __device__ __forceinline__ bool colour_sides(uint32_t* info, const FlowBodies& B
             level[i] = col;
             mx = max(mx, col + 1u);
         }
+    }
     ok = __shfl_sync(full, ok, 0);
     mx = __shfl_sync(full, mx, 0);
     __syncwarp();
@@ -368,21 +372,40 @@ __device__ __forceinline__ uint32_t order_contacts(const uint32_t* info, const F
     return chained;
 }
 
+// The records of a run, in shared memory (or, when they do not fit, in s_rec): word k
+// of all contacts together, even contacts apart from odd ones.  Lanes take neighbouring
+// contacts (contact order) or every other one (a chain's colours), and read 16-byte
+// words without bank conflicts either way; whole records of 160 bytes cost four-way
+// ones, which bound runs with several contacts per lane.
+struct Recs {
+    float4* p;
+    uint32_t half, stride;
+    static constexpr uint32_t kPad = 7;  // contacts' worth of padding at most
+    __device__ __forceinline__ Recs(float4* shared, float4* global, uint32_t nc) {
+        p = shared ? shared : global;
+        half = (nc + 1) / 2;
+        if (shared) half += (12u - half % 8u) % 8u;  // 4 modulo 8
+        stride = half + nc / 2;
+    }
+    __device__ __forceinline__ float4* at(uint32_t i) const { return p + (i >> 1) + (i & 1u) * half; }
+};
+
 struct FlowArgs {
-    uint32_t c0, nc, slot, width, threads, iters;  // nc: chained contacts
-    const uint32_t* order;  // contact (from c0) of each position
+    uint32_t nc, slot, width, threads, iters;  // nc: chained contacts
+    const uint32_t* order;  // contact of each position
     const uint32_t* info;
-    const float4* rec;  // records by contact
+    Recs rec;
+    float* lam;         // impulses by contact
+    uint32_t* deg;      // degrees of both bodies by contact (scratch)
     uint32_t* left;     // lanes that are not done
 };
 
 // The rounds of one bundle's chained contacts.  kSeveral: lanes own more than one.
 template <uint32_t W, bool kSeveral>
-__device__ __forceinline__ void flow_sweep(const World& w, const Scratch& s, const FlowArgs& f,
-                                           const FlowBodies& B) {
+__device__ __forceinline__ void flow_sweep(const FlowArgs& f, const FlowBodies& B) {
     const unsigned full = 0xFFFFFFFFu;
     uint32_t i = f.slot, it = 0, c = f.order[min(i, f.nc - 1)];
-    Rec h = load_rec(f.rec + size_t(c) * kRecWords);
+    Rec h = load_rec(f.rec.at(c), f.rec.stride);
     uint32_t xa = f.info[2 * c], xb = f.info[2 * c + 1];
     uint32_t da = 0, db = 0, ka = 0, kb = 0;  // degrees, counts to wait for
     State x{};
@@ -391,25 +414,28 @@ __device__ __forceinline__ void flow_sweep(const World& w, const Scratch& s, con
     // counts start at the body's contacts (the ranking's result)
     auto arm = [&] {
         if (kSeveral) {
-            const size_t at = size_t(f.c0 + c) * 2;
-            da = s.s_abp[at];
-            db = s.s_abp[at + 1];
+            const uint32_t d = f.deg[c];
+            da = d & 0xFFFFu;
+            db = d >> 16;
         }
         ka = da * (it + 1) + (xa >> kRankShift);
         kb = db * (it + 1) + (xb >> kRankShift);
-        const float4 va = ld4(B.v + (xa & kSideBody)), wa = ld4(B.w + (xa & kSideBody)),
-                     vb = ld4(B.v + (xb & kSideBody)), wb = ld4(B.w + (xb & kSideBody));
-        x.va = mk(va.x, va.y, va.z);
-        x.wa = mk(wa.x, wa.y, wa.z);
-        x.vb = mk(vb.x, vb.y, vb.z);
-        x.wb = mk(wb.x, wb.y, wb.z);
+        if (!kSeveral || (xa & kSideFree)) {  // (the others are read in every round)
+            const float4 v = ld4(B.v + (xa & kSideBody)), o = ld4(B.w + (xa & kSideBody));
+            x.va = mk(v.x, v.y, v.z);
+            x.wa = mk(o.x, o.y, o.z);
+        }
+        if (!kSeveral || (xb & kSideFree)) {
+            const float4 v = ld4(B.v + (xb & kSideBody)), o = ld4(B.w + (xb & kSideBody));
+            x.vb = mk(v.x, v.y, v.z);
+            x.wb = mk(o.x, o.y, o.z);
+        }
     };
     if (kSeveral) {
         // the degrees of the lane's contacts, before the counts move on
         for (uint32_t j = i; j < f.nc; j += f.width) {
             const uint32_t e = f.order[j];
-            s.s_abp[size_t(f.c0 + e) * 2] = degree(f.info[2 * e]);
-            s.s_abp[size_t(f.c0 + e) * 2 + 1] = degree(f.info[2 * e + 1]);
+            f.deg[e] = degree(f.info[2 * e]) | degree(f.info[2 * e + 1]) << 16;
         }
     } else {
         da = degree(xa);
@@ -458,7 +484,7 @@ __device__ __forceinline__ void flow_sweep(const World& w, const Scratch& s, con
                     st4(B.v + lb, make_float4(y.vb.x, y.vb.y, y.vb.z, __uint_as_float(kb + 1u)));
                 }
                 if (kSeveral) {  // on to the lane's next contact
-                    w.lambda[f.c0 + c] = x.lam;
+                    f.lam[c] = x.lam;
                     i += f.width;
                     if (i >= f.nc) {
                         i = f.slot;
@@ -466,10 +492,10 @@ __device__ __forceinline__ void flow_sweep(const World& w, const Scratch& s, con
                     }
                     if (live) {
                         c = f.order[i];
-                        h = load_rec(f.rec + size_t(c) * kRecWords);
+                        h = load_rec(f.rec.at(c), f.rec.stride);
                         xa = f.info[2 * c];
                         xb = f.info[2 * c + 1];
-                        x.lam = w.lambda[f.c0 + c];
+                        x.lam = f.lam[c];
                         arm();
                     }
                 } else {
@@ -483,13 +509,13 @@ __device__ __forceinline__ void flow_sweep(const World& w, const Scratch& s, con
         }
         part_sync<W>(f.threads);
     }
-    if (!kSeveral && i < f.nc) w.lambda[f.c0 + c] = x.lam;
+    if (!kSeveral && i < f.nc) f.lam[c] = x.lam;
 }
 
 // The lone contacts (no other contact at their dynamic bodies): all their
 // iterations at once, 32 contacts per warp, the batches by ticket.
-__device__ __forceinline__ void lone_sweep(const World& w, const FlowArgs& f, const FlowBodies& B,
-                                           uint32_t total, uint32_t* ticket) {
+__device__ __forceinline__ void lone_sweep(const FlowArgs& f, const FlowBodies& B, uint32_t total,
+                                           uint32_t* ticket) {
     const uint32_t lane = threadIdx.x & 31u;
     for (;;) {
         uint32_t b = 0;
@@ -499,7 +525,7 @@ __device__ __forceinline__ void lone_sweep(const World& w, const FlowArgs& f, co
         if (b + lane >= total) continue;
         const uint32_t c = f.order[b + lane], xa = f.info[2 * c], xb = f.info[2 * c + 1];
         if (xa & kSideSkip) continue;
-        const Rec h = load_rec(f.rec + size_t(c) * kRecWords);
+        const Rec h = load_rec(f.rec.at(c), f.rec.stride);
         const uint32_t la = xa & kSideBody, lb = xb & kSideBody;
         const float4 va = ld4(B.v + la), wa = ld4(B.w + la), vb = ld4(B.v + lb), wb = ld4(B.w + lb);
         State x{mk(va.x, va.y, va.z), mk(wa.x, wa.y, wa.z), mk(vb.x, vb.y, vb.z),
@@ -524,8 +550,103 @@ __device__ __forceinline__ void lone_sweep(const World& w, const FlowArgs& f, co
             st4(B.v + lb, make_float4(x.vb.x, x.vb.y, x.vb.z, 0.0f));
             st4(B.w + lb, make_float4(x.wb.x, x.wb.y, x.wb.z, 0.0f));
         }
-        w.lambda[f.c0 + c] = x.lam;
+        f.lam[c] = x.lam;
     }
+}
+
+struct RunShared {
+    uint32_t order, failed, left, chained, ticket;
+};
+
+// The solve of a run of nc contacts by a block of W warps, the bodies' velocities and
+// the sides' words in place, left and ticket zero.  c0: the run's place in the scratch
+// lists; contact(i), body(l): the contact and body that i and l stand for; lam: the
+// impulses, zero before; deg: nc words.  Mode COLORED where a body needs more than 32 colours: contact
+// order, or (fall_back false) nothing is done and the result is false.
+template <uint32_t W, class Contact, class Body>
+__device__ __forceinline__ bool solve_run(const World& w, const Consts& k, const Scratch& s,
+                                          uint32_t mode, float dt, uint32_t c0, uint32_t nc,
+                                          uint32_t nbs, const FlowBodies& B, uint32_t* info,
+                                          uint32_t* order, const Recs& rec, float* lam, uint32_t* deg,
+                                          uint32_t salt,
+                                          bool fall_back, RunShared& sh, Contact contact, Body body) {
+    constexpr uint32_t kThreads = 32 * W;
+    const uint32_t t = threadIdx.x, lane = t & 31u, wid = t >> 5;
+    // ---- ranks and positions by the last warp, records by the others ----
+    if (wid == W - 1) {
+        bool coloured = mode == 2, ok = true;
+        if (coloured && !colour_sides(info, B, nc, deg, s.s_order + c0)) {
+            coloured = false;  // contact order instead
+            for (uint32_t i = lane; i < nbs; i += 32) *B.count(i) = 0;
+            __syncwarp();
+        }
+        if (mode != 0 && !coloured) ok = rank_sides(info, B, nc);
+        if (coloured) {
+            __syncwarp();
+            for (uint32_t i = lane; i < nbs; i += 32) *B.count(i) = __popc(*B.count(i));
+            __syncwarp();
+        }
+        uint32_t chained = 0;
+        if (mode != 0) {
+            __syncwarp();
+            chained = order_contacts(info, B, nc, kThreads, coloured ? s.s_order + c0 : nullptr, order);
+        }
+        // contacts one by one, the reference's loop, when the ranks are too large
+        if (lane == 0) {
+            sh.order = mode != 0 && ok;
+            sh.failed = mode == 2 && !coloured;
+            sh.chained = chained;
+        }
+    }
+    if (W == 1 || wid < W - 1)
+        for (uint32_t i = t; i < nc; i += 32 * (W == 1 ? 1 : W - 1)) {
+            const uint32_t la = info[2 * i] & kSideBody, lb = info[2 * i + 1] & kSideBody;
+            const float4 va = B.v[la], wa = B.w[la], vb = B.v[lb], wb = B.w[lb];
+            make_rec(w, k, contact(i), body(la), body(lb), mk(va.x, va.y, va.z), mk(wa.x, wa.y, wa.z),
+                     mk(vb.x, vb.y, vb.z), mk(wb.x, wb.y, wb.z), dt, rec.at(i), rec.stride);
+        }
+    __syncthreads();
+    if (sh.failed && !fall_back) return false;
+
+    if (!sh.order) {
+        // ---- SEQUENTIAL: the reference order, one lane ----
+        if (t == 0)
+            for (uint32_t it = 0; it < k.pgs_iterations; ++it)
+                for (uint32_t i = 0; i < nc; ++i) {
+                    const uint32_t xa = info[2 * i], xb = info[2 * i + 1];
+                    if (xa & kSideSkip) continue;
+                    const uint32_t la = xa & kSideBody, lb = xb & kSideBody;
+                    const float4 va = B.v[la], wa = B.w[la], vb = B.v[lb], wb = B.w[lb];
+                    const State x = update(load_rec(rec.at(i), rec.stride), true,
+                                           State{mk(va.x, va.y, va.z), mk(wa.x, wa.y, wa.z),
+                                                 mk(vb.x, vb.y, vb.z), mk(wb.x, wb.y, wb.z),
+                                                 lam[i]});
+                    if (!(xa & kSideFree)) {
+                        B.v[la] = make_float4(x.va.x, x.va.y, x.va.z, 0.0f);
+                        B.w[la] = make_float4(x.wa.x, x.wa.y, x.wa.z, 0.0f);
+                    }
+                    if (!(xb & kSideFree)) {
+                        B.v[lb] = make_float4(x.vb.x, x.vb.y, x.vb.z, 0.0f);
+                        B.w[lb] = make_float4(x.wb.x, x.wb.y, x.wb.z, 0.0f);
+                    }
+                    lam[i] = x.lam;
+                }
+    } else {
+        // contacts go to the warps from a different one on in each block, so that
+        // the longest chains of an SM's blocks do not meet on one scheduler
+        const uint32_t role = (wid + salt) % W, chained = sh.chained;
+        const FlowArgs f{chained, role * 32 + lane, kThreads, 32u * min(W, (chained + 31) / 32),
+                         k.pgs_iterations, order, info, rec, lam, deg, &sh.left};
+        if (role * 32 < chained) {  // dataflow rounds, by the warps that own chained contacts
+            if (chained > kThreads)
+                flow_sweep<W, true>(f, B);
+            else
+                flow_sweep<W, false>(f, B);
+        }
+        lone_sweep(f, B, nc, &sh.ticket);
+    }
+    __syncthreads();
+    return true;
 }
 
 // nbmax: bodies of the largest bundle; recs: contact records that fit in shared
@@ -536,11 +657,11 @@ __global__ void __launch_bounds__(32 * W, 12 / W)
                   uint32_t recs) {
     constexpr uint32_t kThreads = 32 * W;
     extern __shared__ float4 sm4[];
-    __shared__ uint32_t sh_order, sh_left, sh_chained, sh_ticket;
+    __shared__ RunShared sh;
     start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;  // contacts from a scan that gave up
-    const uint32_t t = threadIdx.x, lane = t & 31u, wid = t >> 5;
+    const uint32_t t = threadIdx.x;
     const uint32_t bundle = blockIdx.x;
     if (bundle >= w.nbundles) return;
     const uint32_t b0 = w.bundle_off[bundle], b1 = w.bundle_off[bundle + 1];
@@ -553,8 +674,8 @@ __global__ void __launch_bounds__(32 * W, 12 / W)
     // (s_level: the colours of mode 2 are done with when the positions are made)
     uint32_t* order = nc <= kInfoCap ? reinterpret_cast<uint32_t*>(sm4 + 2 * nbmax + kInfoCap / 2)
                                      : s.s_level + c0;
-    float4* rec = nc <= recs ? sm4 + 2 * nbmax + kInfoCap / 2 + kInfoCap / 4
-                             : s.s_rec + size_t(c0) * kRecWords;
+    const Recs rec(nc + Recs::kPad <= recs ? sm4 + 2 * nbmax + kInfoCap / 2 + kInfoCap / 4 : nullptr,
+                   s.s_rec + size_t(c0) * kRecWords, nc);
 
     // ---- the bundle's bodies; every contact side's body and flags ----
     for (uint32_t i = t; i < nc; i += kThreads) {
@@ -579,87 +700,151 @@ __global__ void __launch_bounds__(32 * W, 12 / W)
         B.v[i] = make_float4(v.x, v.y, v.z, 0.0f);
         B.w[i] = make_float4(om.x, om.y, om.z, 0.0f);
     }
-    if (t == 0) sh_left = sh_ticket = 0;
+    if (t == 0) sh.left = sh.ticket = 0;
     __syncthreads();
-
-    // ---- ranks and positions by the last warp, records by the others ----
-    if (wid == W - 1) {
-        bool coloured = mode == 2, ok = true;
-        if (coloured && !colour_sides(info, B, nc, s.s_level + c0, s.s_order + c0)) {
-            coloured = false;  // contact order instead
-            for (uint32_t i = lane; i < nbs; i += 32) *B.count(i) = 0;
-            __syncwarp();
-        }
-        if (mode != 0 && !coloured) ok = rank_sides(info, B, nc);
-        if (coloured) {
-            __syncwarp();
-            for (uint32_t i = lane; i < nbs; i += 32) *B.count(i) = __popc(*B.count(i));
-            __syncwarp();
-        }
-        uint32_t chained = 0;
-        if (mode != 0) {
-            __syncwarp();
-            chained = order_contacts(info, B, nc, kThreads, coloured ? s.s_order + c0 : nullptr, order);
-        }
-        // contacts one by one, the reference's loop, when the ranks are too large
-        if (lane == 0) {
-            sh_order = mode != 0 && ok;
-            sh_chained = chained;
-        }
-    }
-    if (W == 1 || wid < W - 1)
-        for (uint32_t i = t; i < nc; i += 32 * (W == 1 ? 1 : W - 1)) {
-            const uint32_t la = info[2 * i] & kSideBody, lb = info[2 * i + 1] & kSideBody;
-            const float4 va = B.v[la], wa = B.w[la], vb = B.v[lb], wb = B.w[lb];
-            make_rec(w, k, c0 + i, b0 + la, b0 + lb, mk(va.x, va.y, va.z), mk(wa.x, wa.y, wa.z),
-                     mk(vb.x, vb.y, vb.z), mk(wb.x, wb.y, wb.z), dt, rec + size_t(i) * kRecWords);
-        }
-    __syncthreads();
-
-    if (!sh_order) {
-        // ---- SEQUENTIAL: the reference order, one lane ----
-        if (t == 0)
-            for (uint32_t it = 0; it < k.pgs_iterations; ++it)
-                for (uint32_t i = 0; i < nc; ++i) {
-                    const uint32_t xa = info[2 * i], xb = info[2 * i + 1];
-                    if (xa & kSideSkip) continue;
-                    const uint32_t la = xa & kSideBody, lb = xb & kSideBody;
-                    const float4 va = B.v[la], wa = B.w[la], vb = B.v[lb], wb = B.w[lb];
-                    const State x = update(load_rec(rec + size_t(i) * kRecWords), true,
-                                           State{mk(va.x, va.y, va.z), mk(wa.x, wa.y, wa.z),
-                                                 mk(vb.x, vb.y, vb.z), mk(wb.x, wb.y, wb.z),
-                                                 w.lambda[c0 + i]});
-                    if (!(xa & kSideFree)) {
-                        B.v[la] = make_float4(x.va.x, x.va.y, x.va.z, 0.0f);
-                        B.w[la] = make_float4(x.wa.x, x.wa.y, x.wa.z, 0.0f);
-                    }
-                    if (!(xb & kSideFree)) {
-                        B.v[lb] = make_float4(x.vb.x, x.vb.y, x.vb.z, 0.0f);
-                        B.w[lb] = make_float4(x.wb.x, x.wb.y, x.wb.z, 0.0f);
-                    }
-                    w.lambda[c0 + i] = x.lam;
-                }
-    } else {
-        // contacts go to the warps from a different one on in each block, so that
-        // the longest chains of an SM's blocks do not meet on one scheduler
-        const uint32_t role = (wid + bundle) % W, chained = sh_chained;
-        const FlowArgs f{c0,   chained, role * 32 + lane, kThreads, 32u * min(W, (chained + 31) / 32),
-                         k.pgs_iterations, order, info, rec, &sh_left};
-        if (role * 32 < chained) {  // dataflow rounds, by the warps that own chained contacts
-            if (chained > kThreads)
-                flow_sweep<W, true>(w, s, f, B);
-            else
-                flow_sweep<W, false>(w, s, f, B);
-        }
-        lone_sweep(w, f, B, nc, &sh_ticket);
-    }
-    __syncthreads();
+    solve_run<W>(
+        w, k, s, mode, dt, c0, nc, nbs, B, info, order, rec, w.lambda + c0, s.s_abp + c0, bundle,
+        true, sh,
+        [&](uint32_t i) { return c0 + i; }, [&](uint32_t l) { return b0 + l; });
     // ---- velocities back to the bound buffers ----
     for (uint32_t i = t; i < nbs; i += kThreads) {
         const float4 v = B.v[i], om = B.w[i];
         st3(w.vel, b0 + i, mk(v.x, v.y, v.z));
         st3(w.omega, b0 + i, mk(om.x, om.y, om.z));
     }
+}
+
+// ---- runs of islands --------------------------------------------------------
+// Contacts sorted by island (islands.cu): a block takes the islands that start in a
+// window of kIslandWindow sorted contacts and sweeps them as a bundle.  Their bodies
+// are not consecutive: the first contact side that claims a body (s_last, zero before)
+// gives it a slot; a fixed body, which several islands may share, gets one per side.
+// Islands of more than kIslandMost contacts and, in mode COLORED, runs with a body of
+// more than 32 colours are marked in todo and counted in left[1] for the kernel that
+// gives each island a warp (k_solver_island).  left[0]: the windows' ticket.
+//
+// Bound by issue (734 instructions per warp and round) where there are many islands:
+// 1,024 towers of 256 boxes, 61 rounds each, 404 us per substep; a warp per island,
+// swept level by level with the velocities in L2, took 651 us.  A settled pile of 2,601
+// bodies (a chain of 91 rounds) 157 against 252 us.  Four warps, so that three blocks
+// share an SM and a tower's colours of 128 contacts fill a round each.
+constexpr uint32_t kIslandWarps = 4, kIslandSmem = 72 * 1024;
+constexpr uint32_t kIslandWindow = 32 * kIslandWarps;
+static_assert((kIslandMost + kIslandWindow) * 56 + kIslandWindow * 36 + 48 <= kIslandSmem,
+              "a run's sides and bodies must fit");
+static_assert(kIslandMost + 2 * kIslandWindow <= kSideBody, "body field too narrow");
+
+__global__ void __launch_bounds__(32 * kIslandWarps, 12 / kIslandWarps)
+    k_island_flow(World w, Consts k, Scratch s, uint32_t mode, float dt, uint32_t* todo, uint32_t* left) {
+    constexpr uint32_t kThreads = 32 * kIslandWarps;
+    extern __shared__ float4 sm4[];
+    __shared__ RunShared sh;
+    __shared__ uint32_t sh_window, sh_slots;
+    start_dependents();
+    wait_for_previous();
+    if (halted(w.status)) return;
+    const uint32_t t = threadIdx.x;
+    const uint32_t count = *s.isl.count, total = s.isl.start[count];
+    const uint32_t* perm = s.isl.perm;
+    for (;;) {
+        if (t == 0) {
+            sh_window = atomicAdd(&left[0], 1u);
+            sh_slots = sh.left = sh.ticket = 0;
+        }
+        __syncthreads();
+        const uint32_t from = sh_window * kIslandWindow;
+        if (from >= total) return;
+        const uint32_t ia = s.isl.idx[from];
+        uint32_t ib = from + kIslandWindow < total ? s.isl.idx[from + kIslandWindow] : count;
+        const uint32_t p0 = s.isl.start[ia];
+        for (uint32_t i = ia + t; i < ib; i += kThreads) todo[i] = 0;
+        // only the last island can reach past the window
+        if (ib > ia && s.isl.start[ib] - s.isl.start[ib - 1] > kIslandMost) {
+            --ib;
+            __syncthreads();
+            if (t == 0) {
+                todo[ib] = 1;
+                atomicAdd(&left[1], 1u);
+            }
+        }
+        const uint32_t nc = ib > ia ? s.isl.start[ib] - p0 : 0u;
+        if (nc > 0) {
+            uint32_t* info = reinterpret_cast<uint32_t*>(sm4);
+            uint32_t *order = info + 2 * nc, *deg = info + 3 * nc;
+            float* lam = reinterpret_cast<float*>(info + 4 * nc);
+            const uint32_t most = nc + (ib - ia);  // bodies: a tree's, an island, at most
+            float4* const bodies = sm4 + (5 * nc + 3) / 4;
+            const FlowBodies B{bodies, bodies + most};
+            uint32_t* list = reinterpret_cast<uint32_t*>(bodies + 2 * most);
+            const uint32_t used = (5 * nc + 3) / 4 + 2 * most + (most + 3) / 4;
+            const Recs rec((used + (nc + Recs::kPad) * kRecWords) * 16 <= kIslandSmem ? sm4 + used : nullptr,
+                           s.s_rec + size_t(p0) * kRecWords, nc);
+            auto fixed = [&](uint32_t b) {
+                const f3 I = ld3(w.inv_inertia, b);
+                return w.inv_mass[b] == 0.0f && I.x == 0.0f && I.y == 0.0f && I.z == 0.0f;
+            };
+            auto claim = [&](uint32_t b, bool f) {
+                if (!f && atomicCAS(&s.s_last[b], 0u, kNone) != 0u) return 0u;
+                const uint32_t slot = atomicAdd(&sh_slots, 1u);
+                const f3 v = ld3(w.vel, b), om = ld3(w.omega, b);
+                B.v[slot] = make_float4(v.x, v.y, v.z, 0.0f);
+                B.w[slot] = make_float4(om.x, om.y, om.z, 0.0f);
+                list[slot] = f ? b | 0x80000000u : b;
+                if (!f) atomicExch(&s.s_last[b], slot + 1u);
+                return slot;
+            };
+            for (uint32_t i = t; i < nc; i += kThreads) {
+                const uint32_t c = perm[p0 + i];
+                const uint32_t a = w.geom_body[w.c_a[c]], b = w.geom_body[w.c_b[c]];
+                info[2 * i] = claim(a, fixed(a));
+                info[2 * i + 1] = claim(b, fixed(b));
+                lam[i] = 0.0f;
+            }
+            __syncthreads();
+            for (uint32_t i = t; i < nc; i += kThreads) {
+                const uint32_t c = perm[p0 + i];
+                const uint32_t a = w.geom_body[w.c_a[c]], b = w.geom_body[w.c_b[c]];
+                const bool fa = fixed(a), fb = fixed(b);
+                const uint32_t la = fa ? info[2 * i] : __ldcg(&s.s_last[a]) - 1u;
+                const uint32_t lb = fb ? info[2 * i + 1] : __ldcg(&s.s_last[b]) - 1u;
+                info[2 * i] = la | (fa || a == b ? kSideFree : 0u);
+                info[2 * i + 1] = lb | (fb ? kSideFree : 0u);
+            }
+            __syncthreads();
+            const uint32_t slots = sh_slots;
+            const bool done = solve_run<kIslandWarps>(
+                w, k, s, mode, dt, p0, nc, slots, B, info, order, rec, lam, deg, sh_window, false,
+                sh, [&](uint32_t i) { return perm[p0 + i]; },
+                [&](uint32_t l) { return list[l] & 0x7FFFFFFFu; });
+            for (uint32_t l = t; l < slots; l += kThreads) {
+                const uint32_t b = list[l];
+                if (b & 0x80000000u) continue;
+                if (!done) {  // as the warp-per-island kernel expects it
+                    s.s_last[b] = 0;
+                    continue;
+                }
+                const float4 v = B.v[l], om = B.w[l];
+                st3(w.vel, b, mk(v.x, v.y, v.z));
+                st3(w.omega, b, mk(om.x, om.y, om.z));
+            }
+            if (done)
+                for (uint32_t i = t; i < nc; i += kThreads) w.lambda[perm[p0 + i]] = lam[i];
+            else
+                for (uint32_t i = ia + t; i < ib; i += kThreads) {
+                    todo[i] = 1;
+                    atomicAdd(&left[1], 1u);
+                }
+        }
+        __syncthreads();
+    }
+}
+
+int launch_island_flow(const World& w, const Consts& k, const Scratch& s, uint32_t mode, float dt,
+                       uint32_t sms, uint32_t* todo, uint32_t* left, cudaStream_t st) {
+    const uint32_t windows = (w.max_contacts + kIslandWindow - 1) / kIslandWindow;
+    launch_after(k_island_flow, std::min(windows, sms * (12 / kIslandWarps)), 32 * kIslandWarps,
+                 kIslandSmem, st, w, k, s, mode, dt, todo, left);
+    return 1;
 }
 
 constexpr uint32_t kSolverMaxSmem = 160 * 1024;
@@ -674,6 +859,9 @@ cudaError_t init_solver() {
             cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFlowMaxSmem));
         if (e != cudaSuccess) return e;
     }
+    const cudaError_t ei = cudaFuncSetAttribute(
+        k_island_flow, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kIslandSmem));
+    if (ei != cudaSuccess) return ei;
     // opt in to more than 48 KB of dynamic shared memory; done at handle
     // creation so that no attribute call happens during graph capture
     return cudaFuncSetAttribute(k_solver, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -86,20 +86,22 @@ struct Rec {
     float bias, kn, rk, mu, msum;  // rk = 1 / kn, 0 when kn is out of div_by's range
     Side a, b;
 };
-__device__ __forceinline__ Side load_side(const float4* p) {
-    const float4 c = p[0], d = p[1], e = p[2], f = p[3];
+// (Words `stride` apart: 1 in lists of whole records.)
+__device__ __forceinline__ Side load_side(const float4* p, uint32_t stride) {
+    const float4 c = p[0], d = p[stride], e = p[2 * stride], f = p[3 * stride];
     return Side{mk(c.x, c.y, c.z), mk(f.x, f.y, f.z),
                 m3{mk(c.w, d.x, d.y), mk(d.z, d.w, e.x), mk(e.y, e.z, e.w)}, f.w};
 }
-__device__ __forceinline__ void store_side(float4* p, const Side& s) {
+__device__ __forceinline__ void store_side(float4* p, uint32_t stride, const Side& s) {
     p[0] = make_float4(s.r.x, s.r.y, s.r.z, s.R.c0.x);
-    p[1] = make_float4(s.R.c0.y, s.R.c0.z, s.R.c1.x, s.R.c1.y);
-    p[2] = make_float4(s.R.c1.z, s.R.c2.x, s.R.c2.y, s.R.c2.z);
-    p[3] = make_float4(s.I.x, s.I.y, s.I.z, s.m);
+    p[stride] = make_float4(s.R.c0.y, s.R.c0.z, s.R.c1.x, s.R.c1.y);
+    p[2 * stride] = make_float4(s.R.c1.z, s.R.c2.x, s.R.c2.y, s.R.c2.z);
+    p[3 * stride] = make_float4(s.I.x, s.I.y, s.I.z, s.m);
 }
-__device__ __forceinline__ Rec load_rec(const float4* p) {
-    const float4 a = p[0], b = p[1];
-    return Rec{mk(a.x, a.y, a.z), a.w, b.x, b.y, b.z, b.w, load_side(p + 2), load_side(p + 6)};
+__device__ __forceinline__ Rec load_rec(const float4* p, uint32_t stride = 1) {
+    const float4 a = p[0], b = p[stride];
+    return Rec{mk(a.x, a.y, a.z), a.w, b.x, b.y, b.z, b.w, load_side(p + 2 * stride, stride),
+               load_side(p + 6 * stride, stride)};
 }
 
 // Contact c's record: the constants, computed from the pre-solve velocities
@@ -107,7 +109,7 @@ __device__ __forceinline__ Rec load_rec(const float4* p) {
 // quat_to_mat gives at every update of the sweep, built once.
 __device__ __forceinline__ void make_rec(const World& w, const Consts& k, uint32_t c, uint32_t a,
                                          uint32_t b, f3 va, f3 wa, f3 vb, f3 wb, float dt,
-                                         float4* out) {
+                                         float4* out, uint32_t stride = 1) {
     const uint32_t ga = w.c_a[c], gb = w.c_b[c];
     const f3 n = ld3(w.c_normal, c), cp = ld3(w.c_pos, c);
     const Side A{sub(cp, ld3(w.pos, a)), ld3(w.inv_inertia, a), quat_to_mat(w.quat, a), w.inv_mass[a]};
@@ -121,9 +123,9 @@ __device__ __forceinline__ void make_rec(const World& w, const Consts& k, uint32
     const float kn = msum + dot(ran, apply_inv_I(A.R, A.I, ran)) + dot(rbn, apply_inv_I(B.R, B.I, rbn));
     const float rk = kn >= kDivMin && kn <= kDivMax ? recip_of(kn, rcp_approx(kn)) : 0.0f;
     out[0] = make_float4(n.x, n.y, n.z, bias);
-    out[1] = make_float4(kn, rk, sqrtf(w.friction[ga] * w.friction[gb]), msum);
-    store_side(out + 2, A);
-    store_side(out + 6, B);
+    out[stride] = make_float4(kn, rk, sqrtf(w.friction[ga] * w.friction[gb]), msum);
+    store_side(out + 2 * stride, stride, A);
+    store_side(out + 6 * stride, stride, B);
 }
 
 // One update (solve_core's operations in solve_core's order).  kBuiltin: with the
