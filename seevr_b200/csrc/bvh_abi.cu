@@ -83,10 +83,11 @@ seevr_status seevr_bvh_create(const seevr_bvh_bindings* b, uint32_t max_tris, se
     cudaGetDevice(&h->device);
     h->b = *b;
     h->max_tris = max_tris;
-    if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
+    if (init_lbvh() != cudaSuccess ||
+        cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
         cudaGetLastError();
         delete h;
-        set_last_error("cudaStreamCreate failed");
+        set_last_error("cudaFuncSetAttribute or cudaStreamCreate failed");
         return SEEVR_ERR_CUDA;
     }
     *out = h;

@@ -33,7 +33,14 @@ namespace seevr {
 namespace {
 
 constexpr uint32_t kIslandThreads = 128;
-constexpr uint32_t kNoKey = 0xFFFFFFFFu;
+// Sort passes (8 bits each) for roots below nb and, above them, the key of skipped
+// contacts: 2 for 65,535 bodies.
+inline uint32_t key_passes(uint32_t nb) {
+    uint32_t p = 1;
+    while (p < 4 && nb >= (1u << (8 * p)) - 1u) ++p;
+    return p;
+}
+inline uint32_t no_key(uint32_t passes) { return passes < 4 ? (1u << (8 * passes)) - 1u : 0xFFFFFFFFu; }
 
 __device__ __forceinline__ bool body_fixed(const World& w, uint32_t b) {
     return w.inv_mass[b] == 0.0f && w.inv_inertia[size_t(b) * 3] == 0.0f &&
@@ -62,8 +69,15 @@ __device__ __forceinline__ uint32_t find_root(uint32_t* parent, uint32_t x) {
 __global__ void k_island_prep(World w, Scratch s) {
     start_dependents();
     wait_for_previous();
-    if (halted(w.status)) return;
     if (blockIdx.x == 0 && threadIdx.x < 3) s.isl.count[threadIdx.x] = 0;
+    // the sort's histogram and look-back words (the sort runs, on whatever keys there
+    // are, after a wait gave up as well)
+    const uint32_t words = lbvh_status_words(min(w.counters[1], w.max_contacts));
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < words; t += gridDim.x * blockDim.x)
+        s.isl.sort_status[t] = 0;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < 4 * 256; t += gridDim.x * blockDim.x)
+        s.isl.sort_hist[t] = 0;
+    if (halted(w.status)) return;
     for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < w.nb; b += gridDim.x * blockDim.x) {
         s.isl.parent[b] = b;
         s.s_last[b] = 0;
@@ -130,44 +144,41 @@ __global__ void k_island_union(World w, Scratch s) {
     }
 }
 
-__global__ void k_island_keys(World w, Scratch s) {
+__global__ void k_island_keys(World w, Scratch s, uint32_t none) {
     start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t nc = min(w.counters[1], w.max_contacts);
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < w.max_contacts;
-         c += gridDim.x * blockDim.x) {
-        uint32_t key = kNoKey;
-        if (c < nc) {
-            const uint32_t a = w.geom_body[w.c_a[c]], b = w.geom_body[w.c_b[c]];
-            if (!(w.inv_mass[a] == 0.0f && w.inv_mass[b] == 0.0f))
-                key = find_root(s.isl.parent, body_fixed(w, a) ? b : a);
-        }
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
+        uint32_t key = none;
+        const uint32_t a = w.geom_body[w.c_a[c]], b = w.geom_body[w.c_b[c]];
+        if (!(w.inv_mass[a] == 0.0f && w.inv_mass[b] == 0.0f))
+            key = find_root(s.isl.parent, body_fixed(w, a) ? b : a);
         s.isl.keys_in[c] = key;
         s.isl.vals_in[c] = c;
     }
 }
 
-__global__ void k_island_heads(World w, Scratch s) {
+__global__ void k_island_heads(World w, Scratch s, uint32_t none) {
     start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t* k = s.isl.keys_out;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < w.max_contacts;
-         i += gridDim.x * blockDim.x)
-        s.isl.head[i] = (k[i] != kNoKey && (i == 0 || k[i - 1] != k[i])) ? 1u : 0u;
+    const uint32_t nc = min(w.counters[1], w.max_contacts);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x)
+        s.isl.head[i] = (k[i] != none && (i == 0 || k[i - 1] != k[i])) ? 1u : 0u;
 }
 
-__global__ void k_island_starts(World w, Scratch s) {
+__global__ void k_island_starts(World w, Scratch s, uint32_t none) {
     start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t* k = s.isl.keys_out;
-    const uint32_t n = w.max_contacts;
+    const uint32_t n = min(w.counters[1], w.max_contacts);
     const uint32_t count = *s.isl.count;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (s.isl.head[i]) s.isl.start[s.isl.idx[i]] = i;
-        if (k[i] != kNoKey && (i + 1 == n || k[i + 1] == kNoKey)) s.isl.start[count] = i + 1;
+        if (k[i] != none && (i + 1 == n || k[i + 1] == none)) s.isl.start[count] = i + 1;
     }
     if (count == 0 && blockIdx.x == 0 && threadIdx.x == 0) s.isl.start[0] = 0;
 }
@@ -347,17 +358,19 @@ int launch_solver_islands(const World& w, const Consts& k, const Scratch& s, uin
     launch_after(k_island_link, ncb, 256, 0, st, w, s);
     launch_after(k_island_shorten, nbb, 256, 0, st, w, s);
     launch_after(k_island_union, ncb, 256, 0, st, w, s);
-    launch_after(k_island_keys, ncb, 256, 0, st, w, s);
+    const uint32_t passes = key_passes(w.nb), none = no_key(passes);
+    launch_after(k_island_keys, ncb, 256, 0, st, w, s, none);
     LbvhScratch ls{};
     ls.hist = s.isl.sort_hist;
     ls.status = s.isl.sort_status;
     ls.wait_limit = s.wait_limit;
     int n = 5 + lbvh_sort(s.isl.keys_in, s.isl.vals_in, s.isl.keys_tmp, s.isl.vals_tmp,
-                          s.isl.keys_out, s.isl.perm, w.max_contacts, ls, &s.status[0], st);
-    launch_after(k_island_heads, ncb, 256, 0, st, w, s);
-    n += 1 + launch_exclusive_scan(s.isl.head, s.isl.idx, nullptr, w.max_contacts, s.isl.count,
+                          s.isl.keys_out, s.isl.perm, &w.counters[1], w.max_contacts, passes, false, ls,
+                          &s.status[0], st);
+    launch_after(k_island_heads, ncb, 256, 0, st, w, s, none);
+    n += 1 + launch_exclusive_scan(s.isl.head, s.isl.idx, &w.counters[1], w.max_contacts, s.isl.count,
                                    w.max_contacts + 1, 0u, s, st);
-    launch_after(k_island_starts, ncb, 256, 0, st, w, s);
+    launch_after(k_island_starts, ncb, 256, 0, st, w, s, none);
     static int per_sm = 0;
     if (per_sm == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solver_island, kIslandThreads, 0);

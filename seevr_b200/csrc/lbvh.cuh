@@ -18,12 +18,7 @@ struct LbvhScratch {
     uint32_t* vals_sorted;  // [cap] original index of each sorted slot
     uint32_t* hist;         // [4*256]
     uint32_t* status;       // [1 + tiles*256] look-back tile status
-    uint32_t* left;         // [2*cap]
-    uint32_t* right;        // [2*cap]
-    uint32_t* parent;       // [2*cap]
-    uint32_t* flags;        // [cap]
-    float* node_min;        // [2*cap*3]
-    float* node_max;        // [2*cap*3]
+    uint32_t* flags;        // [cap] arrivals at each split of the tree
     // rows of static bodies (body broadphase): list, count and per-block
     // breadth-first work areas (kStaticBlocks x 3 x 2*cap)
     uint32_t* static_list;   // [cap]
@@ -32,7 +27,7 @@ struct LbvhScratch {
     // partners of each dynamic body's row found by the count traversal, in
     // ascending order, for rows of at most kRowCache partners
     uint32_t* row_cache;  // [cap * kRowCache]
-    // the body tree packed for the traversals: node k at [2k, 2k+1]
+    // the body tree, a record per node (lbvh.cu BodyTree): node k at [2k, 2k+1]
     float4* packed;  // [2 * 2*cap]
     // polls of an unpublished sort tile before a look-back gives up
     uint32_t wait_limit = kSpinLimit;
@@ -44,12 +39,7 @@ constexpr uint32_t kStaticBlocks = 8;
 constexpr uint32_t kRowCache = 8;
 
 struct LbvhView {
-    const float* node_min;
-    const float* node_max;
-    const uint32_t* left;
-    const uint32_t* right;
     const uint32_t* vals;
-    // the same tree as one 32-byte record per node (lbvh.cu k_pack_nodes)
     const float4* packed;
 };
 
@@ -69,11 +59,18 @@ struct TriOut {
     uint32_t* flags;       // binding 15
 };
 
-inline uint32_t lbvh_status_words(uint32_t cap) { return 1 + ((cap + 2047) / 2048) * 256; }
+__host__ __device__ constexpr uint32_t lbvh_status_words(uint32_t cap) { return 1 + ((cap + 2047) / 2048) * 256; }
 
+// Sorts the first min(*n_dev, n) pairs (n_dev NULL: n) by the low 8 `passes` bits of
+// their keys.  s.status (lbvh_status_words(n)) and s.hist zero before; counted: s.hist
+// holds the keys' digit counts already.
 int lbvh_sort(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_tmp,
-              uint32_t* vals_tmp, uint32_t* keys_out, uint32_t* vals_out, uint32_t n,
-              const LbvhScratch& s, uint32_t* err, cudaStream_t st);
+              uint32_t* vals_tmp, uint32_t* keys_out, uint32_t* vals_out, const uint32_t* n_dev,
+              uint32_t n, uint32_t passes, bool counted, const LbvhScratch& s, uint32_t* err,
+              cudaStream_t st);
+// Shared-memory limits of the tree kernels on the current device, once per handle (not
+// while a stream is being captured).
+cudaError_t init_lbvh();
 int lbvh_build_bodies(const World& w, const LbvhScratch& s, uint32_t* err, cudaStream_t st);
 int launch_broadphase_lbvh(const World& w, const Scratch& sc, const LbvhScratch& s,
                            cudaStream_t st);

@@ -945,12 +945,7 @@ seevr_status seevr_physics_create(const seevr_bindings* b, const seevr_caps* cap
         ALLOC(lb.vals_sorted, n);
         ALLOC(lb.hist, 4 * 256);
         ALLOC(lb.status, lbvh_status_words(c.max_bodies));
-        ALLOC(lb.left, 2 * n);
-        ALLOC(lb.right, 2 * n);
-        ALLOC(lb.parent, 2 * n);
         ALLOC(lb.flags, n);
-        ALLOC(lb.node_min, 6 * n);
-        ALLOC(lb.node_max, 6 * n);
         ALLOC(lb.static_list, n);
         ALLOC(lb.static_count, 1);
         ALLOC(lb.bfs, size_t(kStaticBlocks) * 3 * 2 * n);
@@ -967,6 +962,8 @@ seevr_status seevr_physics_create(const seevr_bindings* b, const seevr_caps* cap
         (cudaMemset(h->s.status, 0, 16) != cudaSuccess ||
          cudaMemset(h->s.scan_tiles, 0, 8 * size_t(h->s.scan_tiles_cap + LookBack::kHead)) != cudaSuccess))
         st = fail(SEEVR_ERR_CUDA, "cudaMemset failed");
+    if (st == SEEVR_OK && init_lbvh() != cudaSuccess)
+        st = fail(SEEVR_ERR_CUDA, "cudaFuncSetAttribute for the tree failed");
     if (st == SEEVR_OK && init_solver() != cudaSuccess)
         st = fail(SEEVR_ERR_CUDA, "cudaFuncSetAttribute for the solver failed");
     if (st == SEEVR_OK) {

@@ -746,9 +746,10 @@ __global__ void __launch_bounds__(32 * kIslandWarps, 12 / kIslandWarps)
     const uint32_t t = threadIdx.x;
     const uint32_t count = *s.isl.count, total = s.isl.start[count];
     const uint32_t* perm = s.isl.perm;
-    for (;;) {
+    // the first windows by block: few of them lie one to an SM
+    for (bool first = true;; first = false) {
         if (t == 0) {
-            sh_window = atomicAdd(&left[0], 1u);
+            sh_window = first ? blockIdx.x : gridDim.x + atomicAdd(&left[0], 1u);
             sh_slots = sh.left = sh.ticket = 0;
         }
         __syncthreads();

@@ -8,8 +8,8 @@ import numpy as np
 import pytest
 
 from helpers import DT, G, read_back
-from seevr_b200 import (SOLVER_COLORED, SOLVER_SEQUENTIAL, SOLVER_WAVEFRONT, Caps, Data, Physics,
-                        make_params)
+from seevr_b200 import (BROADPHASE_LBVH, SOLVER_COLORED, SOLVER_SEQUENTIAL, SOLVER_WAVEFRONT, Caps,
+                        Data, Physics, make_params)
 
 pytestmark = pytest.mark.gpu
 
@@ -61,9 +61,9 @@ def plates(n):
     return d
 
 
-def run(d, cuda, solver, giant=0, frames=2, pgs=6):
+def run(d, cuda, solver, giant=0, frames=2, pgs=6, broadphase=0):
     buf = d.upload(cuda, Caps.for_data(d))
-    ph = Physics(buf, make_params(pgs_iterations=pgs, solver=solver, flags=4))
+    ph = Physics(buf, make_params(pgs_iterations=pgs, solver=solver, flags=4, broadphase=broadphase))
     if giant:
         ph.set_tuning(giant_island_contacts=giant)
     for _ in range(frames):
@@ -83,6 +83,16 @@ def test_contact_order(cuda, name):
     d = SCENES[name]()
     a, b = run(d, cuda, SOLVER_SEQUENTIAL), run(d, cuda, SOLVER_WAVEFRONT)
     assert a["num_contacts"] > 400
+    for k in KEYS:
+        assert np.array_equal(a[k], b[k], equal_nan=True), k
+
+
+def test_three_sort_passes(cuda):
+    """67,201 bodies: the islands' roots no longer fit two 8-bit digits."""
+    d = Data.towers(seed=0, towers=2100, height=32, spacing=2.0, overlap=0.004)
+    a, b = (run(d, cuda, s, frames=1, broadphase=BROADPHASE_LBVH)
+            for s in (SOLVER_SEQUENTIAL, SOLVER_WAVEFRONT))
+    assert a["num_contacts"] > 60000
     for k in KEYS:
         assert np.array_equal(a[k], b[k], equal_nan=True), k
 
