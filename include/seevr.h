@@ -441,6 +441,23 @@ seevr_status seevr_physics_adjoint_substep(seevr_physics* h, uint32_t num_bodies
                                            const float gravity[3],
                                            const seevr_adjoint_grads* grads);
 
+/* A rollout's substeps in one call each way, without host work in between
+ * (seevr_b200.grad).  seevr_physics_rollout runs `steps` frames of one substep
+ * of dt, ordered on `stream` as seevr_physics_step_async, and writes the state
+ * before each to checkpoints (device, f32[steps][13 * N]: pos, quat, vel,
+ * omega); overflows are reported by seevr_physics_read_flags.
+ * seevr_physics_adjoint_rollout restores the checkpoints in reverse order and
+ * does what seevr_physics_adjoint_substep does for each; statuses are those of
+ * that call, reported after the last substep.  The checkpoints are not
+ * written.  (With checkpoints NULL and steps 1, the bound state is used.) */
+seevr_status seevr_physics_rollout(seevr_physics* h, uint32_t num_bodies, uint32_t num_hull_verts,
+                                   uint32_t steps, float dt, const float gravity[3],
+                                   float* checkpoints, void* stream);
+seevr_status seevr_physics_adjoint_rollout(seevr_physics* h, uint32_t num_bodies,
+                                           uint32_t num_hull_verts, uint32_t steps, float dt,
+                                           const float gravity[3], float* checkpoints,
+                                           const seevr_adjoint_grads* grads);
+
 /* ---- path tracer (raytracer.zig / raytrace.comp) ------------------------- */
 
 /* Binding indices of Raytracer.init (raytracer.zig:31-58), identical to

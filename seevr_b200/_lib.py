@@ -138,6 +138,8 @@ def _load():
         "seevr_physics_kernel_launches": (U64, [P]),
         "seevr_physics_read_lbvh": (I, [P, U32, UP, UP, FP]),
         "seevr_physics_adjoint_substep": (I, [P, U32, U32, F, FP, C.POINTER(AdjointGrads)]),
+        "seevr_physics_rollout": (I, [P, U32, U32, U32, F, FP, P, P]),
+        "seevr_physics_adjoint_rollout": (I, [P, U32, U32, U32, F, FP, P, C.POINTER(AdjointGrads)]),
         "seevr_raytrace": (I, [C.POINTER(RtBindings), C.POINTER(RtParams), P]),
         "seevr_raytrace_fov_scale": (F, []),
         "seevr_physics_step_noalloc": (I, [C.POINTER(Bindings), C.POINTER(Params), U32, U32,

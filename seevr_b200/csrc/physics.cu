@@ -70,10 +70,11 @@ struct GraphKey {
     // host arrays whose copies the frame holds (seevr_physics_step_io), or
     // none
     const void* io[8];
+    bool own_lut;  // the frame finds the lookups' aliases itself
     bool operator==(const GraphKey& o) const {
         for (int i = 0; i < 8; ++i)
             if (io[i] != o.io[i]) return false;
-        return nb == o.nb && nv == o.nv && nhv == o.nhv && substeps == o.substeps && dt == o.dt &&
+        return own_lut == o.own_lut && nb == o.nb && nv == o.nv && nhv == o.nhv && substeps == o.substeps && dt == o.dt &&
                g[0] == o.g[0] && g[1] == o.g[1] && g[2] == o.g[2];
     }
 };
@@ -115,6 +116,8 @@ struct seevr_physics {
     // adjoint work arrays, allocated by the first adjoint call
     AdjScratch adj{};
     bool adj_ready = false;
+    // the support lookups' aliases are those of this call (no frame needs its own)
+    bool lut_done = false;
     // broadphase overlap words (s.bp_mask), sized for the scene layout
     size_t bp_mask_cap = 0;
     // broadphase tile table (s.bp_tiles) capacity, in tiles
@@ -355,6 +358,7 @@ struct FrameIssue {
             wc.nv = render ? nv : 0u;
             n += launch_check_inputs(wc, uint32_t(h->b.bytes[SEEVR_B_SUPPORT_LOOKUP] / 4), st);
         }
+        if (h->lut_done) return;
         const Range r("phys/lut_alias");
         n += launch_lut_alias(w, h->s, st);
     }
@@ -1103,7 +1107,7 @@ seevr_status run_frames(seevr_physics* h, uint32_t num_bodies, uint32_t num_vert
         return SEEVR_OK;
     }
     GraphKey key{num_bodies, num_vertices, num_hull_verts, substeps, dt,
-                 {gravity[0], gravity[1], gravity[2]}, {}};
+                 {gravity[0], gravity[1], gravity[2]}, {}, !h->lut_done};
     if (io) {
         const void* p[8] = {io->pos_in,  io->quat_in,  io->vel_in,  io->omega_in,
                             io->pos_out, io->quat_out, io->vel_out, io->omega_out};
@@ -1322,14 +1326,36 @@ seevr_status seevr_physics_read_lbvh(seevr_physics* h, uint32_t n, uint32_t* mor
     return SEEVR_OK;
 }
 
-seevr_status seevr_physics_adjoint_substep(seevr_physics* h, uint32_t num_bodies,
-                                           uint32_t num_hull_verts, float dt,
-                                           const float gravity[3],
-                                           const seevr_adjoint_grads* grads) {
-    if (!h || !gravity || !grads) return fail(SEEVR_ERR_INVALID_ARGUMENT, "handle, gravity or grads is NULL");
-    if (!grads->pos || !grads->quat || !grads->vel || !grads->omega || !grads->friction)
-        return fail(SEEVR_ERR_INVALID_ARGUMENT, "a gradient buffer is NULL");
-    if (num_bodies == 0) return SEEVR_OK;
+}  // extern "C"
+
+// ---- rollouts ----------------------------------------------------------------
+namespace {
+
+// State rows to (kSave) or from a checkpoint: pos, quat, vel, omega, one after the other.
+template <bool kSave>
+__global__ void k_checkpoint(World w, float* ckpt) {
+    start_dependents();
+    wait_for_previous();
+    const size_t nb = w.nb;
+    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < 13 * nb;
+         i += size_t(gridDim.x) * blockDim.x) {
+        float* x = i < 3 * nb    ? w.pos + i
+                   : i < 7 * nb  ? w.quat + (i - 3 * nb)
+                   : i < 10 * nb ? w.vel + (i - 7 * nb)
+                                 : w.omega + (i - 10 * nb);
+        if (kSave) ckpt[i] = *x; else *x = ckpt[i];
+    }
+}
+
+template <bool kSave>
+int launch_checkpoint(const World& w, float* ckpt, cudaStream_t st) {
+    const uint32_t blocks = uint32_t((size_t(w.nb) * 13 + 255) / 256);
+    k_checkpoint<kSave><<<std::min(blocks, 148u * 8u), 256, 0, st>>>(w, ckpt);
+    return 1;
+}
+
+// The checks of an adjoint call; the work arrays at the first one.
+seevr_status adjoint_begin(seevr_physics* h, uint32_t num_bodies, uint32_t num_hull_verts) {
     if (h->params.narrowphase != SEEVR_NARROWPHASE_MPR)
         return fail(SEEVR_ERR_NOT_SUPPORTED, "the adjoint differentiates the MPR narrowphase only");
     seevr_status st = check_step_args(h, num_bodies, 0, num_hull_verts);
@@ -1368,25 +1394,95 @@ seevr_status seevr_physics_adjoint_substep(seevr_physics* h, uint32_t num_bodies
     w.nhv = num_hull_verts;
     w.ns = h->num_scenes;
     w.nbundles = h->num_bundles;
+    return SEEVR_OK;
+}
+
+// What every substep of a call shares: hull ranges and lookup aliases.
+uint64_t adjoint_shared(seevr_physics* h, cudaStream_t s) {
     uint64_t n = 0;
     if (!h->b.ptr[SEEVR_B_HULL_RANGE])
         n += launch_hull_range_from_geom_data(static_cast<const float*>(h->b.ptr[SEEVR_B_GEOM_DATA]),
-                                              h->s.derived_hull_range, num_bodies, s);
-    // the substep's forward up to its contacts, in the order of issue_frame
-    n += launch_body_stage(w, h->k, kGravity | kAabb, dt, gravity[0], gravity[1], gravity[2], s);
+                                              h->s.derived_hull_range, h->w.nb, s);
+    return n + launch_lut_alias(h->w, h->s, s);
+}
+
+// One substep's forward up to its contacts, in the order of issue_frame, and its reverse.
+uint64_t adjoint_issue(seevr_physics* h, float dt, const float gravity[3],
+                       const seevr_adjoint_grads* grads, cudaStream_t s) {
+    const World& w = h->w;
+    const AdjScratch& a = h->adj;
+    uint64_t n = launch_body_stage(w, h->k, kGravity | kAabb, dt, gravity[0], gravity[1], gravity[2], s);
     n += h->params.broadphase == SEEVR_BROADPHASE_LBVH ? launch_broadphase_lbvh(w, h->s, h->lb, s)
                                                        : launch_broadphase_n2(w, h->s, h->max_scene_bodies, s);
-    n += launch_lut_alias(w, h->s, s);
     n += launch_narrowphase_taped(w, h->k, h->s, a.ptape, a.ctape, s);
     const Grads g{grads->pos, grads->quat, grads->vel, grads->omega, grads->friction};
-    n += launch_adjoint(w, h->k, h->s, a, g, dt, h->max_bundle_bodies, s);
-    h->launches += n;
+    return n + launch_adjoint(w, h->k, h->s, a, g, dt, h->max_bundle_bodies, s);
+}
+
+seevr_status adjoint_end(seevr_physics* h, cudaStream_t s) {
     SEEVR_CUDA(cudaGetLastError());
     bool overflow = false;
-    st = collect_flags(h, s, &overflow);
+    const seevr_status st = collect_flags(h, s, &overflow);
     if (st != SEEVR_OK) return st;
     if (overflow) return fail(SEEVR_ERR_CAPACITY, "pairs or contacts exceeded the caps");
     return SEEVR_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+seevr_status seevr_physics_adjoint_substep(seevr_physics* h, uint32_t num_bodies,
+                                           uint32_t num_hull_verts, float dt,
+                                           const float gravity[3],
+                                           const seevr_adjoint_grads* grads) {
+    return seevr_physics_adjoint_rollout(h, num_bodies, num_hull_verts, 1, dt, gravity, nullptr, grads);
+}
+
+seevr_status seevr_physics_adjoint_rollout(seevr_physics* h, uint32_t num_bodies,
+                                           uint32_t num_hull_verts, uint32_t steps, float dt,
+                                           const float gravity[3], float* checkpoints,
+                                           const seevr_adjoint_grads* grads) {
+    if (!h || !gravity || !grads) return fail(SEEVR_ERR_INVALID_ARGUMENT, "handle, gravity or grads is NULL");
+    if (!grads->pos || !grads->quat || !grads->vel || !grads->omega || !grads->friction)
+        return fail(SEEVR_ERR_INVALID_ARGUMENT, "a gradient buffer is NULL");
+    if (!checkpoints && steps > 1)
+        return fail(SEEVR_ERR_INVALID_ARGUMENT, "several substeps need their checkpoints");
+    if (num_bodies == 0 || steps == 0) return SEEVR_OK;
+    seevr_status st = adjoint_begin(h, num_bodies, num_hull_verts);
+    if (st != SEEVR_OK) return st;
+    const cudaStream_t s = h->stream;
+    uint64_t n = adjoint_shared(h, s);
+    for (uint32_t k = steps; k-- > 0;) {
+        if (checkpoints) n += launch_checkpoint<false>(h->w, checkpoints + size_t(k) * 13 * num_bodies, s);
+        n += adjoint_issue(h, dt, gravity, grads, s);
+    }
+    h->launches += n;
+    return adjoint_end(h, s);
+}
+
+seevr_status seevr_physics_rollout(seevr_physics* h, uint32_t num_bodies, uint32_t num_hull_verts,
+                                   uint32_t steps, float dt, const float gravity[3], float* checkpoints,
+                                   void* stream) {
+    if (!h || !gravity || !checkpoints)
+        return fail(SEEVR_ERR_INVALID_ARGUMENT, "handle, gravity or checkpoints is NULL");
+    if (num_bodies == 0 || steps == 0) return SEEVR_OK;
+    seevr_status st = check_step_args(h, num_bodies, 0, num_hull_verts);
+    if (st != SEEVR_OK) return st;
+    SEEVR_CUDA(cudaSetDevice(h->device));
+    const cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : h->stream;
+    st = ensure_single_scene(h, num_bodies, s);
+    h->w.nb = num_bodies;
+    if (st == SEEVR_OK && h->groups.empty()) {
+        h->launches += launch_lut_alias(h->w, h->s, s);
+        h->lut_done = true;
+    }
+    for (uint32_t k = 0; k < steps && st == SEEVR_OK; ++k) {
+        h->launches += launch_checkpoint<true>(h->w, checkpoints + size_t(k) * 13 * num_bodies, s);
+        st = run_frames(h, num_bodies, 0, num_hull_verts, 1, dt, gravity, 1, s, nullptr);
+    }
+    h->lut_done = false;
+    return st;
 }
 
 const char* seevr_status_string(seevr_status s) {

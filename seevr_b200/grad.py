@@ -10,10 +10,10 @@
 The forward runs the regular step one substep at a time (a frame of k
 substeps is exactly k calls of one substep with dt / k), ordered on the
 current stream, and keeps a checkpoint of (pos, quat, vel, omega) before
-each.  The backward restores
-each checkpoint in reverse order and calls seevr_physics_adjoint_substep,
-which recomputes that substep's contacts and PGS sweep on the GPU and
-propagates dL/d(state) back through it, accumulating dL/d friction.
+each (seevr_physics_rollout).  The backward restores
+each checkpoint in reverse order, recomputes that substep's contacts and PGS
+sweep on the GPU and propagates dL/d(state) back through it, accumulating
+dL/d friction (seevr_physics_adjoint_rollout).
 Contact selection and the solver's clamps are piecewise constant, so the
 gradient is that of the branch the forward took.  No counterpart in the
 reference, whose step has no reverse mode.
@@ -57,11 +57,12 @@ class _Rollout:
                     t["geom_friction"][:nb].copy_(friction.detach().reshape(-1))
                     # checkpoints and substeps stay ordered on one stream,
                     # with no host round trip until the end
-                    stream = torch.cuda.current_stream(ph.buffers.device)
-                    ckpt = []
-                    for _ in range(steps):
-                        ckpt.append(torch.cat([v.clone() for v in views]))
-                        ph.step_async(nb, 0, nhv, 1, sub_dt, gravity, frames=1, stream=stream)
+                    stream = torch.cuda.current_stream(ph.buffers.device).cuda_stream
+                    ckpt = torch.empty(max(steps, 1), 13 * max(nb, 1), device=ph.buffers.device)
+                    # (torch's default stream is CUDA's legacy default stream, 1)
+                    L.check(L.lib.seevr_physics_rollout(ph._h, nb, nhv, steps, sub_dt,
+                                                        L.fptr(gravity, 3), ckpt.data_ptr(),
+                                                        C.c_void_p(stream or 1)))
                     outs = [v.clone().reshape(x.shape) for v, x in zip(views, ins)]
                     torch.cuda.synchronize(ph.buffers.device)
                     if ph.read_flags() & (L.DEVICE_FLAG_PAIR_OVERFLOW | L.DEVICE_FLAG_CONTACT_OVERFLOW):
@@ -85,15 +86,10 @@ class _Rollout:
                 gf = torch.zeros(max(nb, 1), dtype=torch.float64, device=dev)
                 gr = L.AdjointGrads(g[0].data_ptr(), g[1].data_ptr(), g[2].data_ptr(),
                                     g[3].data_ptr(), gf.data_ptr())
-                views = [t[name][: nb * k] for name, k in _names()]
-                sizes = [nb * k for _, k in _names()]
-                with torch.no_grad():
-                    for ck in reversed(ctx.ckpt):
-                        for v, part in zip(views, torch.split(ck, sizes)):
-                            v.copy_(part)
-                        torch.cuda.current_stream(dev).synchronize()
-                        L.check(L.lib.seevr_physics_adjoint_substep(
-                            ph._h, nb, nhv, sub_dt, L.fptr(gravity, 3), C.byref(gr)))
+                torch.cuda.current_stream(dev).synchronize()
+                L.check(L.lib.seevr_physics_adjoint_rollout(
+                    ph._h, nb, nhv, steps, sub_dt, L.fptr(gravity, 3), ctx.ckpt.data_ptr(),
+                    C.byref(gr)))
                 ctx.ckpt = None
                 sh = ctx.shapes
                 f = lambda x, shape: x.reshape(shape).to(torch.float32)
