@@ -605,7 +605,7 @@ def towers_leg(a, rank, world, dev):
     return {"unit": UNIT, "bodies": nb, "towers": a.towers, "height": h,
             "overlap_m": a.tower_overlap, "substeps": a.substeps,
             "pgs_iterations": a.pgs, "broadphase": "LBVH",
-            "solver_work": "islands: a warp each, islands above 4,096 contacts grid-wide "
+            "solver_work": "islands: runs of them in a block each, islands above 4,096 contacts grid-wide "
                            "(coloured order)",
             "contact_model": "one MPR contact per touching pair (physics.comp:475-491)",
             "note": "PGS passes support one box up a stack per iteration: 256-box towers sink "
@@ -688,21 +688,21 @@ NCU_METRICS = ("gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.su
 NCU_CAPTURED = {"bodies": 123288, "pairs": 118480, "contacts": 28231}
 NCU_CAPTURE = {
     "phys/aabb": {"kernel": "k_body_stage", "skip": 1001, "scale": "bodies",
-                  "dram_bytes_per_launch": 247286528, "duration_us": 60.2,
-                  "issue_active_pct": 44.7, "warps_active_pct": 38.1, "lanes_per_inst": 27.9,
+                  "dram_bytes_per_launch": 247142272, "duration_us": 54.0,
+                  "issue_active_pct": 51.9, "warps_active_pct": 42.9, "lanes_per_inst": 27.9,
                   "registers": 64},
     "phys/broad_phase": {"kernel": "k_broad_tile<0> + k_broad_tile<1>", "skip": 1820,
                          "scale": "bodies", "dram_bytes_per_launch": 10507520,
                          "duration_us": 56.8, "issue_active_pct": 40.5,
                          "warps_active_pct": 56.3, "lanes_per_inst": 29.5, "registers": 63},
     "phys/narrow_phase": {"kernel": "k_narrow<0, 7>", "skip": 910, "scale": "pairs",
-                          "dram_bytes_per_launch": 96512384, "duration_us": 128.1,
-                          "issue_active_pct": 33.5, "warps_active_pct": 32.8,
+                          "dram_bytes_per_launch": 94348288, "duration_us": 122.0,
+                          "issue_active_pct": 34.9, "warps_active_pct": 33.3,
                           "lanes_per_inst": 8.1, "registers": 72},
-    "phys/pgs_solve": {"kernel": "k_solver_warp", "skip": 910, "scale": "bodies",
-                       "dram_bytes_per_launch": 10583040, "duration_us": 286.9,
-                       "issue_active_pct": 9.1, "warps_active_pct": 2.8, "lanes_per_inst": 16.2,
-                       "registers": 141},
+    "phys/pgs_solve": {"kernel": "k_solver_flow", "skip": 910, "scale": "bodies",
+                       "dram_bytes_per_launch": 10580224, "duration_us": 193.9,
+                       "issue_active_pct": 16.1, "warps_active_pct": 11.1, "lanes_per_inst": 28.4,
+                       "registers": 168},
     "phys/render_verts": {"kernel": "k_render_verts", "skip": 91, "scale": "bodies",
                           "dram_bytes_per_launch": 394073344, "duration_us": 98.7,
                           "issue_active_pct": 35.3, "warps_active_pct": 39.8,
@@ -735,7 +735,7 @@ def roofline(stage_ms, ms_per_step, nb, nhv, nv, pairs, contacts, substeps, peak
         "phys/narrow_phase": ("k_narrow (+ scan, scatter)", "latency: dependent gathers, "
                               "divergence", 64 * pairs + 36 * contacts),
         "phys/clear_impulse": ("memset", "hbm", 4 * contacts),
-        "phys/pgs_solve": ("k_solver_warp", "latency: dependent chain of the largest bundle",
+        "phys/pgs_solve": ("k_solver_flow", "latency: dependent chain of the largest bundle",
                            100 * nb + 44 * contacts),
     }
     once = {"phys/render_verts": ("k_render_verts", "hbm", 28 * nb + 24 * nv)}

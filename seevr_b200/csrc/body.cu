@@ -137,7 +137,6 @@ __global__ void __launch_bounds__(kBodyThreads) k_body_stage(World w, Consts k, 
     __shared__ float sh_pose[kBodyThreads][12];  // p xyz, R by columns
     __shared__ uint32_t sh_body[kBodyThreads];
     __shared__ uint32_t sh_n;
-    start_dependents();
     wait_for_previous();
     if (check_failed(w.status)) return;  // bounds-check mode: hull ranges not valid
     if (threadIdx.x == 0) sh_n = 0;

@@ -39,7 +39,6 @@ template <bool kWrite>
 __global__ void __launch_bounds__(256) k_broad_n2(World w, const uint32_t* __restrict__ row_off,
                                                   uint32_t* __restrict__ row_count,
                                                   uint32_t* __restrict__ mask, uint32_t stride) {
-    start_dependents();
     wait_for_previous();
     if (kWrite && halted(w.status)) return;  // row offsets from a scan that gave up
     const uint32_t lane = threadIdx.x & 31u;
@@ -95,7 +94,6 @@ __global__ void __launch_bounds__(kTileThreads)
                  const uint32_t* __restrict__ row_off, uint32_t* __restrict__ row_count,
                  uint32_t* __restrict__ mask, uint32_t stride) {
     extern __shared__ float sm[];
-    start_dependents();
     wait_for_previous();
     if (kWrite && halted(w.status)) return;  // row offsets from a scan that gave up
     uint32_t scene, slice, slices;

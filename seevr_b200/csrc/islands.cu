@@ -67,7 +67,6 @@ __device__ __forceinline__ uint32_t find_root(uint32_t* parent, uint32_t x) {
 // Every island kernel runs on contacts from the narrowphase's scan (and the
 // later ones on the island sort): none runs after a wait gave up.
 __global__ void k_island_prep(World w, Scratch s) {
-    start_dependents();
     wait_for_previous();
     if (blockIdx.x == 0 && threadIdx.x < 3) s.isl.count[threadIdx.x] = 0;
     // the sort's histogram and look-back words (the sort runs, on whatever keys there
@@ -94,7 +93,6 @@ __device__ __forceinline__ bool joins(const World& w, uint32_t c, uint32_t& a, u
 }
 
 __global__ void k_island_link(World w, Scratch s) {
-    start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t nc = min(w.counters[1], w.max_contacts);
@@ -107,7 +105,6 @@ __global__ void k_island_link(World w, Scratch s) {
 // Every body's link to its root.  A body takes over its parent's link, while that
 // body does the same, so the links' lengths double; each step goes to a smaller index.
 __global__ void k_island_shorten(World w, Scratch s) {
-    start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;
     volatile uint32_t* p = s.isl.parent;
@@ -123,7 +120,6 @@ __global__ void k_island_shorten(World w, Scratch s) {
 // Hook the roots of a contact's two dynamic bodies: a failed CAS returns a
 // smaller root, so every retry makes progress.
 __global__ void k_island_union(World w, Scratch s) {
-    start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t nc = min(w.counters[1], w.max_contacts);
@@ -145,7 +141,6 @@ __global__ void k_island_union(World w, Scratch s) {
 }
 
 __global__ void k_island_keys(World w, Scratch s, uint32_t none) {
-    start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t nc = min(w.counters[1], w.max_contacts);
@@ -160,7 +155,6 @@ __global__ void k_island_keys(World w, Scratch s, uint32_t none) {
 }
 
 __global__ void k_island_heads(World w, Scratch s, uint32_t none) {
-    start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t* k = s.isl.keys_out;
@@ -170,7 +164,6 @@ __global__ void k_island_heads(World w, Scratch s, uint32_t none) {
 }
 
 __global__ void k_island_starts(World w, Scratch s, uint32_t none) {
-    start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t* k = s.isl.keys_out;
@@ -188,7 +181,6 @@ __global__ void k_island_starts(World w, Scratch s, uint32_t none) {
 __global__ void __launch_bounds__(kIslandThreads)
     k_solver_island(World w, Consts k, Scratch s, uint32_t mode, float dt, uint32_t giant,
                     const uint32_t* __restrict__ todo) {
-    start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;
     if (todo && s.isl.count[2] == 0) return;

@@ -70,7 +70,6 @@ __global__ void k_body_centroids(const float* __restrict__ aabb_min,
                                  const float* __restrict__ aabb_max, uint32_t n,
                                  float* __restrict__ centroid, uint32_t* bounds_o, SortState sort) {
     __shared__ uint32_t smn[3], smx[3];
-    start_dependents();
     sort.clear();
     if (threadIdx.x < 3) {
         smn[threadIdx.x] = 0xFFFFFFFFu;
@@ -101,7 +100,6 @@ __global__ void k_tri_centroids(const float* __restrict__ verts, const uint32_t*
                                 uint32_t n, float* __restrict__ centroid, uint32_t* bounds_o,
                                 SortState sort) {
     __shared__ uint32_t smn[3], smx[3];
-    start_dependents();
     sort.clear();
     if (threadIdx.x < 3) {
         smn[threadIdx.x] = 0xFFFFFFFFu;
@@ -158,7 +156,6 @@ __global__ void k_sort_counts(const uint32_t* __restrict__ keys, const uint32_t*
                               uint32_t* __restrict__ hist) {
     __shared__ uint32_t sh[4 * kRadix];
     const DigitCounts counts{sh};
-    start_dependents();
     wait_for_previous();
     const uint32_t n = n_dev ? min(*n_dev, n_cap) : n_cap;
     if (blockIdx.x * blockDim.x >= n) return;
@@ -189,7 +186,6 @@ __global__ void __launch_bounds__(kSortThreads)
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp_hist[kSortWarps][kRadix];
     __shared__ uint32_t s_bin_off[kRadix], s_bins[kRadix / 32];
-    start_dependents();
     wait_for_previous();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, shift = 8 * pass;
     const uint32_t n = n_dev ? min(*n_dev, n_cap) : n_cap;
@@ -421,7 +417,6 @@ __global__ void k_morton(const float* __restrict__ centroid, uint32_t n,
                          uint32_t* __restrict__ hist) {
     __shared__ uint32_t sh[4 * kRadix];
     const DigitCounts counts{sh};
-    start_dependents();
     wait_for_previous();
     counts.clear();
     __syncthreads();
@@ -562,7 +557,6 @@ __global__ void __launch_bounds__(kTreeThreads)
     __shared__ signed char s_delta[kTreeThreads + 1];
     __shared__ uint2 s_left[kMostLeft];
     __shared__ uint32_t s_nleft;
-    start_dependents();
     wait_for_previous();
     if (halted(err)) return;  // the sort gave up: the keys are not ordered
     const uint32_t t = threadIdx.x, first = blockIdx.x * kTreeThreads, i = first + t;
@@ -750,7 +744,6 @@ __global__ void __launch_bounds__(256)
                        const uint32_t* static_list, const uint32_t* static_count, uint32_t* bfs) {
     extern __shared__ uint32_t bits[];
     __shared__ uint32_t sh_next, sh_found, sh_cur, sh_warp[8];
-    start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;  // the tree (or the row offsets) are not valid
     const uint32_t n = w.nb;

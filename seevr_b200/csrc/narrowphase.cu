@@ -455,7 +455,6 @@ __global__ void __launch_bounds__(kNarrowThreads, kMinBlocks)
              const uint32_t* __restrict__ order) {
     __shared__ float wit[4][Witness<kTape>::kWords][kNarrowThreadsW];
     __shared__ float pose[2][12][kNarrowThreadsW];
-    start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;  // pairs from a scan that gave up
     const uint32_t np = min(w.counters[0], w.max_pairs);
@@ -907,7 +906,6 @@ __global__ void k_contact_scatter(World w, const float4* __restrict__ res0,
                                   const uint32_t* __restrict__ coff,
                                   const uint4* __restrict__ pair_tape,
                                   uint4* __restrict__ contact_tape, uint32_t* ticket) {
-    start_dependents();
     wait_for_previous();
     if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0u;  // the narrowphase's
     if (halted(w.status)) return;  // offsets from a scan that gave up

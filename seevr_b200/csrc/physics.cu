@@ -1334,7 +1334,6 @@ namespace {
 // State rows to (kSave) or from a checkpoint: pos, quat, vel, omega, one after the other.
 template <bool kSave>
 __global__ void k_checkpoint(World w, float* ckpt) {
-    start_dependents();
     wait_for_previous();
     const size_t nb = w.nb;
     for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < 13 * nb;

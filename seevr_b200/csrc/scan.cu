@@ -24,7 +24,6 @@ __global__ void __launch_bounds__(kScanThreads)
            LookBack lb, uint32_t* status) {
     __shared__ uint32_t s_tile, s_excl, s_tag;
     __shared__ uint32_t s_warp[kScanThreads / 32];
-    start_dependents();
     wait_for_previous();
     const uint32_t n = n_dev ? min(*n_dev, n_cap) : n_cap;
     const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;

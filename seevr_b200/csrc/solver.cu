@@ -658,7 +658,6 @@ __global__ void __launch_bounds__(32 * W, 12 / W)
     constexpr uint32_t kThreads = 32 * W;
     extern __shared__ float4 sm4[];
     __shared__ RunShared sh;
-    start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;  // contacts from a scan that gave up
     const uint32_t t = threadIdx.x;
@@ -740,7 +739,6 @@ __global__ void __launch_bounds__(32 * kIslandWarps, 12 / kIslandWarps)
     extern __shared__ float4 sm4[];
     __shared__ RunShared sh;
     __shared__ uint32_t sh_window, sh_slots;
-    start_dependents();
     wait_for_previous();
     if (halted(w.status)) return;
     const uint32_t t = threadIdx.x;
