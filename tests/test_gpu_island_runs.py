@@ -2,7 +2,7 @@
 against the sequential loop, in colour order against the warp-per-island kernel
 (which a giant-island threshold of 1,024 contacts selects).  Islands of one
 contact, below, at and above a run's window of 128 contacts, above the 1,024
-contacts a run takes, and a body with more than 32 contacts (no 32 colours)
+contacts a run takes (128 in contact order), and a body with more than 32 contacts (no 32 colours)
 among others in one run."""
 import numpy as np
 import pytest
