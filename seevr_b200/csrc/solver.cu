@@ -209,9 +209,11 @@ __global__ void __launch_bounds__(kSolverThreads)
 // head of its lane's list and ready, so every round makes progress.
 constexpr uint32_t kInfoCap = 512;  // contacts whose bodies, ranks and positions fit in smem
 // a contact side's bundle-local body, flags and rank
-// (Free: the body is not written and orders nothing; Skip: both masses infinite)
-constexpr uint32_t kSideBody = 0xFFFu, kSideFree = 1u << 12, kSideSkip = 1u << 13, kRankShift = 16,
-                   kMaxRank = 0xFFFFu;
+// (Free: the body is not written and orders nothing; Skip: both masses infinite;
+// Same, with Free, on side a: side b is the same dynamic body, whose velocities
+// side a reads at every update and which b writes last)
+constexpr uint32_t kSideBody = 0xFFFu, kSideFree = 1u << 12, kSideSkip = 1u << 13,
+                   kSideSame = 1u << 14, kRankShift = 16, kMaxRank = 0xFFFFu;
 static_assert(kWarpMaxBodies <= kSideBody, "body field too narrow");
 
 // Shared memory of a block: per body its velocity with the count of its updates
@@ -420,7 +422,8 @@ __device__ __forceinline__ void flow_sweep(const FlowArgs& f, const FlowBodies& 
         }
         ka = da * (it + 1) + (xa >> kRankShift);
         kb = db * (it + 1) + (xb >> kRankShift);
-        if (!kSeveral || (xa & kSideFree)) {  // (the others are read in every round)
+        // (the others are read in every round, and so is a body that is both sides)
+        if ((!kSeveral || (xa & kSideFree)) && !(xa & kSideSame)) {
             const float4 v = ld4(B.v + (xa & kSideBody)), o = ld4(B.w + (xa & kSideBody));
             x.va = mk(v.x, v.y, v.z);
             x.wa = mk(o.x, o.y, o.z);
@@ -463,6 +466,10 @@ __device__ __forceinline__ void flow_sweep(const FlowArgs& f, const FlowBodies& 
             ready = ready && __float_as_uint(v.w) == kb;
             x.vb = mk(v.x, v.y, v.z);
             x.wb = mk(o.x, o.y, o.z);
+        }
+        if (xa & kSideSame) {
+            x.va = x.vb;
+            x.wa = x.wb;
         }
         const uint32_t left = *f.left;
         part_sync<W>(f.threads);  // every read of the round before its writes
@@ -531,6 +538,10 @@ __device__ __forceinline__ void lone_sweep(const FlowArgs& f, const FlowBodies& 
         State x{mk(va.x, va.y, va.z), mk(wa.x, wa.y, wa.z), mk(vb.x, vb.y, vb.z),
                 mk(wb.x, wb.y, wb.z), 0.0f};
         for (uint32_t it = 0; it < f.iters; ++it) {
+            if (xa & kSideSame) {
+                x.va = x.vb;
+                x.wa = x.wb;
+            }
             const State y = update(h, true, x);
             x.lam = y.lam;
             if (!(xa & kSideFree)) {  // a fixed body keeps its velocities
@@ -688,8 +699,9 @@ __global__ void __launch_bounds__(32 * W, 12 / W)
             xa |= kSideSkip | kSideFree;
             xb |= kSideSkip | kSideFree;
         } else {
-            if (fa || a == b) xa |= kSideFree;  // both sides one body: b is written last
+            if (fa) xa |= kSideFree;
             if (fb) xb |= kSideFree;
+            if (a == b && !fb) xa |= kSideFree | kSideSame;
         }
         info[2 * i] = xa;
         info[2 * i + 1] = xb;
@@ -809,7 +821,7 @@ __global__ void __launch_bounds__(32 * kIslandWarps, 12 / kIslandWarps)
                 const bool fa = fixed(a), fb = fixed(b);
                 const uint32_t la = fa ? info[2 * i] : __ldcg(&s.s_last[a]) - 1u;
                 const uint32_t lb = fb ? info[2 * i + 1] : __ldcg(&s.s_last[b]) - 1u;
-                info[2 * i] = la | (fa || a == b ? kSideFree : 0u);
+                info[2 * i] = la | (fa ? kSideFree : 0u) | (a == b && !fb ? kSideFree | kSideSame : 0u);
                 info[2 * i + 1] = lb | (fb ? kSideFree : 0u);
             }
             __syncthreads();
