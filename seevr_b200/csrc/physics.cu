@@ -1473,7 +1473,11 @@ seevr_status seevr_physics_rollout(seevr_physics* h, uint32_t num_bodies, uint32
     st = ensure_single_scene(h, num_bodies, s);
     h->w.nb = num_bodies;
     if (st == SEEVR_OK && h->groups.empty()) {
-        h->launches += launch_lut_alias(h->w, h->s, s);
+        // the lookups' aliases once, after what a frame does before them: the hull
+        // ranges they read, and in bounds-check mode the checks of both
+        FrameIssue f(h, num_bodies, 0, num_hull_verts, 1, dt, gravity, s, nullptr);
+        f.begin();
+        h->launches += f.n;
         h->lut_done = true;
     }
     for (uint32_t k = 0; k < steps && st == SEEVR_OK; ++k) {
