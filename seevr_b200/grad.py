@@ -58,7 +58,8 @@ class _Rollout:
                     # checkpoints and substeps stay ordered on one stream,
                     # with no host round trip until the end
                     stream = torch.cuda.current_stream(ph.buffers.device).cuda_stream
-                    ckpt = torch.empty(max(steps, 1), 13 * max(nb, 1), device=ph.buffers.device)
+                    ckpt = torch.empty(max(steps, 1), 13 * max(nb, 1), dtype=torch.float32,
+                                       device=ph.buffers.device)
                     # (torch's default stream is CUDA's legacy default stream, 1)
                     L.check(L.lib.seevr_physics_rollout(ph._h, nb, nhv, steps, sub_dt,
                                                         L.fptr(gravity, 3), ckpt.data_ptr(),
