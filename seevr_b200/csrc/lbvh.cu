@@ -288,8 +288,12 @@ __global__ void __launch_bounds__(kSortThreads)
         if (i < n) {
             const uint32_t d = (key[k] >> shift) & 0xFFu;
             const uint32_t dst = s_bin_off[d] + s_warp_hist[warp][d] + rank[k];
-            keys_out[dst] = key[k];
-            vals_out[dst] = val[k];
+            // (after a pass that gave up, slots hold keys that the histogram does not
+            // count, whose digits run past the end)
+            if (dst < n) {
+                keys_out[dst] = key[k];
+                vals_out[dst] = val[k];
+            }
         }
     }
 }
