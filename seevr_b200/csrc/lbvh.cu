@@ -562,7 +562,10 @@ __global__ void __launch_bounds__(kTreeThreads)
     __shared__ uint2 s_left[kMostLeft];
     __shared__ uint32_t s_nleft;
     wait_for_previous();
-    if (halted(err)) return;  // the sort gave up: the keys are not ordered
+    // the sort gave up: the keys are not ordered.  (One answer for the block: another
+    // block's wait below may give up meanwhile, and what a part of the block left out
+    // the rest would read.)
+    if (__syncthreads_or(halted(err) ? 1 : 0)) return;
     const uint32_t t = threadIdx.x, first = blockIdx.x * kTreeThreads, i = first + t;
     const uint32_t here = min(kTreeThreads, n - first);
     uint32_t *s_key = tsm, *s_met = tsm + kTreeThreads;

@@ -1,7 +1,8 @@
 """A sort whose look-backs give up (wait limit 0): the step ends with a timeout and
 stays within its buffers, and the handle, its limit restored, steps like a fresh one.
 The body tree's sort (30-bit codes, four passes) and the islands' (two and three
-passes)."""
+passes); and a tree of more blocks than run at once, where a wait of the first ones
+gives up while others begin."""
 import numpy as np
 import pytest
 
@@ -14,7 +15,7 @@ pytestmark = pytest.mark.gpu
 ROWS = ("body_pos", 3), ("body_quat", 4), ("body_vel", 3), ("body_omega", 3)
 
 
-@pytest.mark.parametrize("towers, height", [(200, 60), (1200, 60)])
+@pytest.mark.parametrize("towers, height", [(200, 60), (1200, 60), (5200, 60)])
 def test_sorts_that_give_up(cuda, towers, height):
     import torch
 
