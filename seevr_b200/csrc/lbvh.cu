@@ -324,6 +324,15 @@ constexpr uint32_t kUnset = 0xFFA5C3E1u;  // a NaN that no arithmetic makes
 __device__ __forceinline__ bool arrived(float x) { return __float_as_uint(x) != kUnset; }
 __device__ __forceinline__ float read_now(const float* p) { return *reinterpret_cast<const volatile float*>(p); }
 
+// A caller's vertex may hold any bits: kUnset becomes the quiet NaN of its payload, so
+// that no box is taken for one that has not arrived.
+__device__ __forceinline__ float unmark(float x) {
+    return arrived(x) ? x : __uint_as_float(kUnset | 0x00400000u);
+}
+__device__ __forceinline__ f3 unmark(f3 v) {
+    return mk(unmark(v.x), unmark(v.y), unmark(v.z));
+}
+
 // Length of the common prefix of the codes at positions i < n - 1 and i + 1, ties by
 // position.
 __device__ __forceinline__ int delta(uint32_t a, uint32_t b, uint32_t i) {
@@ -345,7 +354,7 @@ struct TriTree {
         const uint32_t pi = vals[i];
         const f3 v0 = ld3(verts, idx[size_t(pi) * 3]), v1 = ld3(verts, idx[size_t(pi) * 3 + 1]),
                  v2 = ld3(verts, idx[size_t(pi) * 3 + 2]);
-        return Box{vmin(vmin(v0, v1), v2), vmax(vmax(v0, v1), v2)};
+        return Box{unmark(vmin(vmin(v0, v1), v2)), unmark(vmax(vmax(v0, v1), v2))};
     }
     __device__ __forceinline__ void leaf(uint32_t i, uint32_t node, const Box& b) const {
         if (o.prim_idx) o.prim_idx[i] = vals[i];
