@@ -178,7 +178,10 @@ __global__ void k_island_starts(World w, Scratch s, uint32_t none) {
 
 // Warp per island (persistent).  Positions p in [start, start+1) index the
 // island's contacts in index order (perm[p] = contact).
-__global__ void __launch_bounds__(kIslandThreads)
+// (Five blocks per SM: left to itself the compiler takes 80 registers, with spills in
+// the sweep, for a sixth.  2,500 boxes in one heap, 44.5 ms per frame with six, 40.4
+// with five; 1,024 towers of 256 boxes in contact order 107.0 and 103.7.)
+__global__ void __launch_bounds__(kIslandThreads, 5)
     k_solver_island(World w, Consts k, Scratch s, uint32_t mode, float dt, uint32_t giant,
                     const uint32_t* __restrict__ todo) {
     wait_for_previous();
