@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(kSolverThreads)
 // A lane owns contacts i, i + 32 W, ... and takes them in order, iteration after
 // iteration: the first unfinished update of the whole sequence is then at the
 // head of its lane's list and ready, so every round makes progress.
-constexpr uint32_t kInfoCap = 512;  // contacts whose bodies, ranks and positions fit in smem
+
 // a contact side's bundle-local body, flags and rank
 // (Free: the body is not written and orders nothing; Skip: both masses infinite;
 // Same, with Free, on side a: side b is the same dynamic body, whose velocities
@@ -217,11 +217,8 @@ constexpr uint32_t kSideBody = 0xFFFu, kSideFree = 1u << 12, kSideSkip = 1u << 1
 static_assert(kWarpMaxBodies <= kSideBody, "body field too narrow");
 
 // Shared memory of a block: per body its velocity with the count of its updates
-// and its angular velocity (a float4 each), the contact sides' words, and records
-// of `recs` contacts for pairs that own several.
-__host__ __device__ constexpr uint32_t flow_smem_bytes(uint32_t nbmax, uint32_t recs) {
-    return 32 * nbmax + 12 * kInfoCap + 16 * kRecWords * recs;
-}
+// and its angular velocity (a float4 each); then, where they fit, the contacts'
+// sides and positions (12 bytes each) and their records.
 struct FlowBodies {
     float4* v;  // velocity, updates counted (bits of an integer)
     float4* w;  // angular velocity, unused
@@ -660,12 +657,10 @@ __device__ __forceinline__ bool solve_run(const World& w, const Consts& k, const
     return true;
 }
 
-// nbmax: bodies of the largest bundle; recs: contact records that fit in shared
-// memory.
+// room: float4s of shared memory, two for every body of the largest bundle at least.
 template <uint32_t W>
 __global__ void __launch_bounds__(32 * W, 12 / W)
-    k_solver_flow(World w, Consts k, Scratch s, uint32_t mode, float dt, uint32_t nbmax,
-                  uint32_t recs) {
+    k_solver_flow(World w, Consts k, Scratch s, uint32_t mode, float dt, uint32_t room) {
     constexpr uint32_t kThreads = 32 * W;
     extern __shared__ float4 sm4[];
     __shared__ RunShared sh;
@@ -678,13 +673,15 @@ __global__ void __launch_bounds__(32 * W, 12 / W)
     const uint32_t c0 = first_contact(w, s, b0), c1 = first_contact(w, s, b1);
     if (c0 >= c1) return;
     const uint32_t nbs = b1 - b0, nc = c1 - c0;
-    const FlowBodies B{sm4, sm4 + nbmax};
-    uint32_t* info = nc <= kInfoCap ? reinterpret_cast<uint32_t*>(sm4 + 2 * nbmax)
-                                    : s.s_ab + size_t(c0) * 2;
+    const FlowBodies B{sm4, sm4 + nbs};
+    uint32_t at = 2 * nbs;
+    const uint32_t lists = (12 * nc + 15) / 16;
+    const bool near = at + lists <= room;
+    uint32_t* info = near ? reinterpret_cast<uint32_t*>(sm4 + at) : s.s_ab + size_t(c0) * 2;
     // (s_level: the colours of mode 2 are done with when the positions are made)
-    uint32_t* order = nc <= kInfoCap ? reinterpret_cast<uint32_t*>(sm4 + 2 * nbmax + kInfoCap / 2)
-                                     : s.s_level + c0;
-    const Recs rec(nc + Recs::kPad <= recs ? sm4 + 2 * nbmax + kInfoCap / 2 + kInfoCap / 4 : nullptr,
+    uint32_t* order = near ? info + 2 * nc : s.s_level + c0;
+    if (near) at += lists;
+    const Recs rec(at + (nc + Recs::kPad) * kRecWords <= room ? sm4 + at : nullptr,
                    s.s_rec + size_t(c0) * kRecWords, nc);
 
     // ---- the bundle's bodies; every contact side's body and flags ----
@@ -862,7 +859,7 @@ int launch_island_flow(const World& w, const Consts& k, const Scratch& s, uint32
 }
 
 constexpr uint32_t kSolverMaxSmem = 160 * 1024;
-constexpr uint32_t kFlowMaxSmem = 120 * 1024;
+constexpr uint32_t kFlowMaxSmem = 120 * 1024, kFlowSmem = 192 * 1024;
 
 cudaError_t init_solver() {
     for (const void* f : {reinterpret_cast<const void*>(k_solver_flow<1>),
@@ -885,23 +882,31 @@ cudaError_t init_solver() {
 // Warps per block by the largest bundle: a settled pile has about a quarter
 // contact per body, two thirds of them chained, and the warps without chained
 // contacts take the lone ones.  Solver time per substep with 1 / 2 / 4 warps:
-// 1,024 scenes in 512-body bundles 274 / 226 / 183 us (295 us before), one
-// 512-body scene - / 162 / 124 us (208 us before).  Above 512 bodies a lane pair
-// of warps more keeps a lane for every chained contact.
+// 1,024 scenes in 512-body bundles 274 / 226 / 183 us, one 512-body scene
+// - / 162 / 124 us.  Above 512 bodies eight warps keep a lane for most chained
+// contacts but take an SM each, so more bundles than SMs, or scene groups (whose other
+// kernels run beside), get four: 4,096 scenes in 1,024-body bundles 471 us with eight,
+// 341 with four, and with eight groups 11.7 and 10.5 ms per frame; one scene of 1,000
+// bodies 1.92 ms per frame with eight, 2.13 with four.
+//
+// Blocks of up to four warps share an SM as its registers allow (twelve warps), with an
+// equal part each of 192 KB of shared memory, of which the system takes a block's first
+// KB.  With 228 KB two blocks of four warps fitted (77,824 bytes each, 454 us for 4,096
+// scenes in 512-body bundles; 377 with three), and three of 76,700 bytes leave the SM's
+// other kernels next to no L1: with eight groups 13.4 ms per frame, 11.2 with 192 KB.
 static void launch_flow(const World& w, const Consts& k, const Scratch& s, uint32_t mode, float dt,
                         uint32_t nbmax, cudaStream_t st) {
-    const uint32_t warps = nbmax <= 128 ? 1u : nbmax <= 256 ? 2u : nbmax <= 512 ? 4u : 8u;
-    // three blocks of four warps share an SM (registers): a third of its shared
-    // memory each, and records that do not fit go to global memory
-    const uint32_t budget = std::min(kFlowMaxSmem, 19456u * warps);
-    const uint32_t base = flow_smem_bytes(nbmax, 0);
-    const uint32_t recs = budget > base ? (budget - base) / (16 * kRecWords) : 0u;
-    const uint32_t smem = flow_smem_bytes(nbmax, recs);
+    const uint32_t warps = nbmax <= 128                                            ? 1u
+                           : nbmax <= 256                                          ? 2u
+                           : nbmax <= 512 || w.nbundles > 148u || s.order_pairs != 0 ? 4u
+                                                                                   : 8u;
+    const uint32_t part = warps <= 4 ? kFlowSmem / (12 / warps) - 1024u - 128u : kFlowMaxSmem;
+    const uint32_t smem = std::max(part, 32 * nbmax) & ~15u;
     switch (warps) {
-        case 1: launch_after(k_solver_flow<1>, w.nbundles, 32, smem, st, w, k, s, mode, dt, nbmax, recs); break;
-        case 2: launch_after(k_solver_flow<2>, w.nbundles, 64, smem, st, w, k, s, mode, dt, nbmax, recs); break;
-        case 4: launch_after(k_solver_flow<4>, w.nbundles, 128, smem, st, w, k, s, mode, dt, nbmax, recs); break;
-        default: launch_after(k_solver_flow<8>, w.nbundles, 256, smem, st, w, k, s, mode, dt, nbmax, recs);
+        case 1: launch_after(k_solver_flow<1>, w.nbundles, 32, smem, st, w, k, s, mode, dt, smem / 16); break;
+        case 2: launch_after(k_solver_flow<2>, w.nbundles, 64, smem, st, w, k, s, mode, dt, smem / 16); break;
+        case 4: launch_after(k_solver_flow<4>, w.nbundles, 128, smem, st, w, k, s, mode, dt, smem / 16); break;
+        default: launch_after(k_solver_flow<8>, w.nbundles, 256, smem, st, w, k, s, mode, dt, smem / 16);
     }
 }
 
