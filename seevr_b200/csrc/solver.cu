@@ -201,12 +201,13 @@ __global__ void __launch_bounds__(kSolverThreads)
 // warp's latency and issue.  So a lane owns a contact for the whole solve, its
 // constants in registers; velocities and counts live in shared memory, both in
 // one 16-byte word per body; and the update's square root and divisions are
-// the branch-free ones of vmath.cuh: a warp where an argument is outside their
+// the branch-free ones of vmath.cuh: a lane with an argument outside their
 // ranges redoes the update with the built-in ones.
 //
 // A lane owns contacts i, i + 32 W, ... and takes them in order, iteration after
 // iteration: the first unfinished update of the whole sequence is then at the
-// head of its lane's list and ready, so every round makes progress.
+// head of its lane's list and ready, so every round makes progress.  (More than two
+// contacts per lane in contact order go level by level instead: level_sweep.)
 
 // a contact side's bundle-local body, flags and rank
 // (Free: the body is not written and orders nothing; Skip: both masses infinite;
@@ -221,9 +222,12 @@ static_assert(kWarpMaxBodies <= kSideBody, "body field too narrow");
 // sides and positions (12 bytes each) and their records.
 struct FlowBodies {
     float4* v;  // velocity, updates counted (bits of an integer)
-    float4* w;  // angular velocity, unused
+    float4* w;  // angular velocity, latest level (zero but while contacts are ordered)
     __device__ __forceinline__ uint32_t* count(uint32_t l) const {
         return reinterpret_cast<uint32_t*>(&v[l].w);
+    }
+    __device__ __forceinline__ uint32_t* last(uint32_t l) const {
+        return reinterpret_cast<uint32_t*>(&w[l].w);
     }
 };
 
@@ -327,30 +331,42 @@ __device__ __forceinline__ bool colour_sides(uint32_t* info, const FlowBodies& B
     return true;
 }
 
-// Positions: first the contacts that share a dynamic body with another one
-// (their count is returned), then the lone ones.  With a lane for each (at most
-// `lanes`), the former go by falling degree (the larger of the two bodies'), so
-// that the longest chains share few warps; lanes that own several need the
-// sequence's order, which `seq` gives (NULL: contact order).  One warp.
-__device__ __forceinline__ uint32_t order_contacts(const uint32_t* info, const FlowBodies& B,
-                                                   uint32_t nc, uint32_t lanes, const uint32_t* seq,
-                                                   uint32_t* order) {
-    const unsigned full = 0xFFFFFFFFu;
+// Contacts per lane above which blocks of several warps sweep contact order level by
+// level (level_sweep).  Lanes that own several take them in turn, and where contacts
+// that follow each other wait for each other (boxes heaped row by row, columns) few
+// lanes find theirs ready.  Solver time per substep in rounds / by levels (the former
+// passes by level, 32 wide): 1,024 scenes of 8 to 500 boxes heaped, 1.4 contacts per body,
+// 2,850 / 1,475 us (1,559); 300 heaps of 120 boxes 1,006 / 549 (874); 64 scenes of 10
+// columns of 48 1,983 / 1,093 (1,406).  Up to two contacts per lane, rounds are the
+// better where chains' iterations follow each other closely: two columns of 125 boxes
+// 280 / 2,426 us, 13 of 10 121 / 249; at worst 20 of 10 314 / 239.  One warp takes as
+// long for a level as for a round (heaps of 90 boxes 391 us in rounds, 507 by levels).
+constexpr uint32_t kSweepFrom = 2;
+
+// The larger of the numbers of contacts at contact i's dynamic bodies (after ranking).
+__device__ __forceinline__ uint32_t degree_of(const uint32_t* info, const FlowBodies& B, uint32_t i) {
+    const uint32_t a = info[2 * i], b = info[2 * i + 1];
+    return max(a & kSideFree ? 0u : *B.count(a & kSideBody), b & kSideFree ? 0u : *B.count(b & kSideBody));
+}
+// Contacts that share a dynamic body with another one.  One warp.
+__device__ __forceinline__ uint32_t count_chained(const uint32_t* info, const FlowBodies& B, uint32_t nc) {
     const uint32_t lane = threadIdx.x & 31u;
-    auto degree = [&](uint32_t i) {
-        const uint32_t a = info[2 * i], b = info[2 * i + 1];
-        return max(a & kSideFree ? 0u : *B.count(a & kSideBody),
-                   b & kSideFree ? 0u : *B.count(b & kSideBody));
-    };
     uint32_t chained = 0;
     for (uint32_t i0 = 0; i0 < nc; i0 += 32)
-        chained += __popc(__ballot_sync(full, i0 + lane < nc && degree(min(i0 + lane, nc - 1)) > 1u));
+        chained += __popc(__ballot_sync(0xFFFFFFFFu, i0 + lane < nc &&
+                                                         degree_of(info, B, min(i0 + lane, nc - 1)) > 1u));
+    return chained;
+}
+
+// Positions: first the chained contacts, then the lone ones.  With a lane for each (at
+// most `lanes`), the former go by falling degree (the larger of the two bodies'), so
+// that the longest chains share few warps; lanes that own several need the
+// sequence's order, which `seq` gives (NULL: contact order).  One warp.
+__device__ __forceinline__ void order_contacts(const uint32_t* info, const FlowBodies& B, uint32_t nc,
+                                               uint32_t chained, uint32_t lanes, const uint32_t* seq,
+                                               uint32_t* order) {
+    const uint32_t lane = threadIdx.x & 31u;
     // classes: degrees 4 and above, 3, 2, lone ones; or all chained ones, lone ones
-    // one warp alone runs the lone ones in the same rounds
-    if (lanes == 32u && nc <= lanes) {
-        if (lane < nc) order[lane] = lane;
-        return nc;
-    }
     const bool one_each = chained <= lanes;
     uint32_t pos = 0;
     for (uint32_t cls = 4; cls > 0; --cls) {
@@ -358,36 +374,100 @@ __device__ __forceinline__ uint32_t order_contacts(const uint32_t* info, const F
         for (uint32_t i0 = 0; i0 < nc; i0 += 32) {
             const bool valid = i0 + lane < nc;
             const uint32_t i = valid ? (!one_each && seq ? seq[i0 + lane] : i0 + lane) : 0u;
-            const uint32_t d = degree(i);
+            const uint32_t d = degree_of(info, B, i);
             const bool hit = valid && (cls == 1u   ? d <= 1u
                                        : !one_each ? d > 1u
                                        : cls == 4u ? d >= 4u
                                                    : d == cls);
-            const unsigned m = __ballot_sync(full, hit);
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, hit);
             if (hit) order[pos + __popc(m & ((1u << lane) - 1u))] = i;
             pos += __popc(m);
         }
     }
-    return chained;
 }
 
-// The records of a run, in shared memory (or, when they do not fit, in s_rec): word k
-// of all contacts together, even contacts apart from odd ones.  Lanes take neighbouring
-// contacts (contact order) or every other one (a chain's colours), and read 16-byte
-// words without bank conflicts either way; whole records of 160 bytes cost four-way
-// ones, which bound runs with several contacts per lane.
-struct Recs {
-    float4* p;
-    uint32_t half, stride;
-    static constexpr uint32_t kPad = 7;  // contacts' worth of padding at most
-    __device__ __forceinline__ Recs(float4* shared, float4* global, uint32_t nc) {
-        p = shared ? shared : global;
-        half = (nc + 1) / 2;
-        if (shared) half += (12u - half % 8u) % 8u;  // 4 modulo 8
-        stride = half + nc / 2;
-    }
-    __device__ __forceinline__ float4* at(uint32_t i) const { return p + (i >> 1) + (i & 1u) * half; }
+// The chained contacts by levels (a contact's is the first after those of the earlier
+// contacts at its dynamic bodies), then the lone ones, and the levels cut into chunks of
+// up to 32.  The whole block; placed: nc words of scratch; counts: two words, zero
+// before, as the bodies' `last` words are, which count the contacts placed at each.
+// (The first contact not yet placed can be: every round places some.)
+struct Chunks {
+    uint32_t *first, *level;  // of each
+    uint32_t n, levels;
 };
+template <uint32_t W>
+__device__ __forceinline__ Chunks build_levels(const uint32_t* info, const FlowBodies& B, uint32_t nc,
+                                               uint32_t chained, uint32_t* placed, uint32_t* order,
+                                               Chunks chunks, uint32_t* counts) {
+    const uint32_t t = threadIdx.x;
+    for (uint32_t i = t; i < nc; i += 32 * W) {
+        const bool lone = degree_of(info, B, i) <= 1u;
+        if (lone) order[chained + atomicAdd(&counts[1], 1u)] = i;
+        placed[i] = lone ? 1u : 0u;
+    }
+    uint32_t from = 0, l = 0;
+    chunks.n = 0;
+    for (; from < chained; ++l) {
+        for (uint32_t i = t; i < nc; i += 32 * W) {
+            if (placed[i]) continue;
+            const uint32_t xa = info[2 * i], xb = info[2 * i + 1];
+            if (!(xa & kSideFree) && *B.last(xa & kSideBody) != xa >> kRankShift) continue;
+            if (!(xb & kSideFree) && *B.last(xb & kSideBody) != xb >> kRankShift) continue;
+            order[atomicAdd(&counts[0], 1u)] = i;
+            placed[i] = 2u + l;
+        }
+        __syncthreads();
+        const uint32_t to = counts[0], n = (to - from + 31) / 32;
+        for (uint32_t j = t; j < n; j += 32 * W) {
+            chunks.first[chunks.n + j] = from + 32 * j;
+            chunks.level[chunks.n + j] = l;
+        }
+        for (uint32_t i = t; i < nc; i += 32 * W) {  // no two of a level share a dynamic body
+            if (placed[i] != 2u + l) continue;
+            const uint32_t xa = info[2 * i], xb = info[2 * i + 1];
+            if (!(xa & kSideFree)) ++*B.last(xa & kSideBody);
+            if (!(xb & kSideFree)) ++*B.last(xb & kSideBody);
+        }
+        __syncthreads();
+        from = to;
+        chunks.n += n;
+    }
+    chunks.levels = l;
+    return chunks;
+}
+
+// The records of a run.  In shared memory word k of all contacts lies together, even
+// contacts apart from odd ones: lanes take neighbouring contacts (contact order) or
+// every other one (a chain's colours), and read 16-byte words without bank conflicts
+// either way; whole records of 160 bytes cost four-way ones, which bound runs with
+// several contacts per lane.  Those that do not fit lie whole in s_rec, five sectors
+// each, and `stage`, where there is room for it, holds `slots` of them at a time for the
+// level sweep.
+struct Recs {
+    float4 *p, *stage;
+    uint32_t half, stride, step, slots;
+    static constexpr uint32_t kPad = 7;  // contacts' worth of padding at most
+    // room: float4s of shared memory; most: threads
+    __device__ __forceinline__ Recs(float4* shared, uint32_t room, float4* global, uint32_t nc, uint32_t most) {
+        const bool fits = (nc + kPad) * kRecWords <= room;
+        p = fits ? shared : global;
+        half = (nc + 1) / 2;
+        half = fits ? half + (12u - half % 8u) % 8u : kRecWords;  // 4 modulo 8
+        stride = fits ? half + nc / 2 : 1u;
+        step = fits ? 1u : 2 * kRecWords;
+        slots = fits ? 0u : min(room / kRecWords & ~31u, most);
+        stage = shared;
+    }
+    __device__ __forceinline__ float4* at(uint32_t i) const {
+        return p + size_t(i >> 1) * step + (i & 1u) * half;
+    }
+};
+__device__ __forceinline__ void copy_async(float4* to, const float4* from) {  // global to shared
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(uint32_t(__cvta_generic_to_shared(to))),
+                 "l"(__cvta_generic_to_global(from))
+                 : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 struct FlowArgs {
     uint32_t nc, slot, width, threads, iters;  // nc: chained contacts
@@ -516,6 +596,104 @@ __device__ __forceinline__ void flow_sweep(const FlowArgs& f, const FlowBodies& 
     if (!kSeveral && i < f.nc) f.lam[c] = x.lam;
 }
 
+// The chained contacts, a level at a time (a turn): its contacts touch different dynamic
+// bodies and run together.  A turn takes 1,100 to 1,400 cycles: the bodies' velocities,
+// the update's chain, the barrier.  The warps take the iterations' chunks in rotation, so
+// that a warp prepares its next chunk (table, contact, sides, record: 400 cycles) while
+// others solve theirs, behind the barrier that ended its own; only where that chunk's
+// turn is this one or the next it starts the record's copy before it solves.
+template <uint32_t W>
+__device__ __forceinline__ void level_sweep(const FlowArgs& f, const FlowBodies& B, const Chunks& chunks) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const bool staged = threadIdx.x < f.rec.slots;
+    float4* const slot = f.rec.stage + threadIdx.x;
+    // a chunk of this warp's: its turn (kNone: none), this lane's contact and its sides
+    struct Part {
+        uint32_t turn, c, xa, xb;
+    };
+    // chunks this far along: the table's entries, then the contacts, then the sides
+    uint32_t at = threadIdx.x >> 5, base = 0;  // chunk of the table read next; its iteration's first turn
+    uint32_t first = 0, end = 0, turn = kNone;
+    auto read_table = [&] {
+        while (at >= chunks.n) {
+            at -= chunks.n;
+            base += chunks.levels;
+        }
+        turn = base + chunks.level[at];
+        first = chunks.first[at];
+        end = min(first + 32u, at + 1 < chunks.n ? chunks.first[at + 1] : f.nc);
+        at += W;
+    };
+    auto read_part = [&] {
+        Part p{turn, kNone, 0u, 0u};
+        if (first + lane < end) p.c = f.order[first + lane];
+        return p;
+    };
+    auto read_sides = [&](Part& p) {
+        if (p.c == kNone) return;
+        p.xa = f.info[2 * p.c];
+        p.xb = f.info[2 * p.c + 1];
+    };
+    auto fetch = [&](uint32_t c) {
+        if (c == kNone || !staged) return;
+        const float4* from = f.rec.at(c);
+#pragma unroll
+        for (uint32_t j = 0; j < kRecWords; ++j) copy_async(slot + j * f.rec.slots, from + j);
+    };
+    const uint32_t turns = f.iters * chunks.levels;
+    read_table();
+    Part cur = read_part();
+    read_table();
+    Part next = read_part();
+    read_table();
+    read_sides(cur);
+    read_sides(next);
+    Rec h{};
+    if (cur.c != kNone) h = load_rec(f.rec.at(cur.c), f.rec.stride);
+    auto advance = [&] {  // cur <- next
+        cur = next;
+        next = read_part();
+        read_sides(next);
+        read_table();
+    };
+    for (uint32_t k = 0; k < turns; ++k) {
+        bool later = false;  // the next chunk's record is still to be loaded
+        while (cur.turn == k) {
+            const bool soon = next.turn <= k + 1;
+            if (soon) fetch(next.c);
+            if (cur.c != kNone) {
+                const uint32_t la = cur.xa & kSideBody, lb = cur.xb & kSideBody;
+                const float4 va = ld4(B.v + la), wa = ld4(B.w + la), vb = ld4(B.v + lb), wb = ld4(B.w + lb);
+                const State y = update(h, true,
+                                       State{mk(va.x, va.y, va.z), mk(wa.x, wa.y, wa.z),
+                                             mk(vb.x, vb.y, vb.z), mk(wb.x, wb.y, wb.z), f.lam[cur.c]});
+                if (!(cur.xa & kSideFree)) {
+                    st4(B.v + la, make_float4(y.va.x, y.va.y, y.va.z, 0.0f));
+                    st4(B.w + la, make_float4(y.wa.x, y.wa.y, y.wa.z, 0.0f));
+                }
+                if (!(cur.xb & kSideFree)) {
+                    st4(B.v + lb, make_float4(y.vb.x, y.vb.y, y.vb.z, 0.0f));
+                    st4(B.w + lb, make_float4(y.wb.x, y.wb.y, y.wb.z, 0.0f));
+                }
+                f.lam[cur.c] = y.lam;
+            }
+            if (!soon) {
+                later = true;
+                break;
+            }
+            advance();
+            copies_done();
+            if (cur.c != kNone)
+                h = staged ? load_rec(slot, f.rec.slots) : load_rec(f.rec.at(cur.c), f.rec.stride);
+        }
+        part_sync<W>(32 * W);
+        if (later) {
+            advance();
+            if (cur.c != kNone) h = load_rec(f.rec.at(cur.c), f.rec.stride);
+        }
+    }
+}
+
 // The lone contacts (no other contact at their dynamic bodies): all their
 // iterations at once, 32 contacts per warp, the batches by ticket.
 __device__ __forceinline__ void lone_sweep(const FlowArgs& f, const FlowBodies& B, uint32_t total,
@@ -563,7 +741,7 @@ __device__ __forceinline__ void lone_sweep(const FlowArgs& f, const FlowBodies& 
 }
 
 struct RunShared {
-    uint32_t order, failed, left, chained, ticket;
+    uint32_t order, failed, left, chained, by_level, placed[2], ticket;
 };
 
 // The solve of a run of nc contacts by a block of W warps, the bodies' velocities and
@@ -594,16 +772,26 @@ __device__ __forceinline__ bool solve_run(const World& w, const Consts& k, const
             for (uint32_t i = lane; i < nbs; i += 32) *B.count(i) = __popc(*B.count(i));
             __syncwarp();
         }
-        uint32_t chained = 0;
+        uint32_t chained = nc;
+        bool by_level = false;
         if (mode != 0) {
             __syncwarp();
-            chained = order_contacts(info, B, nc, kThreads, coloured ? s.s_order + c0 : nullptr, order);
+            if (kThreads == 32u && nc <= kThreads) {  // the warp runs the lone ones in the same rounds
+                if (lane < nc) order[lane] = lane;
+            } else {
+                chained = count_chained(info, B, nc);
+                by_level = W > 1 && ok && !coloured && chained > kSweepFrom * kThreads;
+                if (!by_level)
+                    order_contacts(info, B, nc, chained, kThreads, coloured ? s.s_order + c0 : nullptr, order);
+            }
         }
         // contacts one by one, the reference's loop, when the ranks are too large
         if (lane == 0) {
             sh.order = mode != 0 && ok;
             sh.failed = mode == 2 && !coloured;
             sh.chained = chained;
+            sh.by_level = by_level;
+            sh.placed[0] = sh.placed[1] = 0;
         }
     }
     if (W == 1 || wid < W - 1)
@@ -615,6 +803,11 @@ __device__ __forceinline__ bool solve_run(const World& w, const Consts& k, const
         }
     __syncthreads();
     if (sh.failed && !fall_back) return false;
+    Chunks chunks{s.s_order + c0, s.s_lvl_start + c0, 0u, 0u};
+    if (W > 1 && sh.by_level) {
+        chunks = build_levels<W>(info, B, nc, sh.chained, deg, order, chunks, sh.placed);
+        __syncthreads();
+    }
 
     if (!sh.order) {
         // ---- SEQUENTIAL: the reference order, one lane ----
@@ -646,7 +839,9 @@ __device__ __forceinline__ bool solve_run(const World& w, const Consts& k, const
         const FlowArgs f{chained, role * 32 + lane, kThreads, 32u * min(W, (chained + 31) / 32),
                          k.pgs_iterations, order, info, rec, lam, deg, &sh.left};
         if (role * 32 < chained) {  // dataflow rounds, by the warps that own chained contacts
-            if (chained > kThreads)
+            if (W > 1 && sh.by_level)
+                level_sweep<W>(f, B, chunks);
+            else if (chained > kThreads)
                 flow_sweep<W, true>(f, B);
             else
                 flow_sweep<W, false>(f, B);
@@ -681,8 +876,7 @@ __global__ void __launch_bounds__(32 * W, 12 / W)
     // (s_level: the colours of mode 2 are done with when the positions are made)
     uint32_t* order = near ? info + 2 * nc : s.s_level + c0;
     if (near) at += lists;
-    const Recs rec(at + (nc + Recs::kPad) * kRecWords <= room ? sm4 + at : nullptr,
-                   s.s_rec + size_t(c0) * kRecWords, nc);
+    const Recs rec(sm4 + at, room - at, s.s_rec + size_t(c0) * kRecWords, nc, kThreads);
 
     // ---- the bundle's bodies; every contact side's body and flags ----
     for (uint32_t i = t; i < nc; i += kThreads) {
@@ -788,8 +982,7 @@ __global__ void __launch_bounds__(32 * kIslandWarps, 12 / kIslandWarps)
             const FlowBodies B{bodies, bodies + most};
             uint32_t* list = reinterpret_cast<uint32_t*>(bodies + 2 * most);
             const uint32_t used = (5 * nc + 3) / 4 + 2 * most + (most + 3) / 4;
-            const Recs rec((used + (nc + Recs::kPad) * kRecWords) * 16 <= kIslandSmem ? sm4 + used : nullptr,
-                           s.s_rec + size_t(p0) * kRecWords, nc);
+            const Recs rec(sm4 + used, kIslandSmem / 16 - used, s.s_rec + size_t(p0) * kRecWords, nc, kThreads);
             auto fixed = [&](uint32_t b) {
                 const f3 I = ld3(w.inv_inertia, b);
                 return w.inv_mass[b] == 0.0f && I.x == 0.0f && I.y == 0.0f && I.z == 0.0f;
