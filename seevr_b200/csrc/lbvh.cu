@@ -189,7 +189,12 @@ __global__ void __launch_bounds__(kSortThreads)
     wait_for_previous();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, shift = 8 * pass;
     const uint32_t n = n_dev ? min(*n_dev, n_cap) : n_cap;
-    if (threadIdx.x == 0) s_tile = atomicAdd(status, 1u) - pass * gridDim.x;
+    if (threadIdx.x == 0) {
+        const uint32_t ticket = atomicAdd(status, 1u) - pass * gridDim.x;
+        // no pass after one that gave up: slots it left unwritten hold keys that the
+        // histogram does not count, and their digits' places run past the end
+        s_tile = halted(err) ? kNone : ticket;
+    }
     // the digit's first slot: exclusive scan of the histogram (a digit per thread)
     const uint32_t digits = threadIdx.x < kRadix ? hist[pass * kRadix + threadIdx.x] : 0u;
     uint32_t bin = digits;
@@ -288,12 +293,8 @@ __global__ void __launch_bounds__(kSortThreads)
         if (i < n) {
             const uint32_t d = (key[k] >> shift) & 0xFFu;
             const uint32_t dst = s_bin_off[d] + s_warp_hist[warp][d] + rank[k];
-            // (after a pass that gave up, slots hold keys that the histogram does not
-            // count, whose digits run past the end)
-            if (dst < n) {
-                keys_out[dst] = key[k];
-                vals_out[dst] = val[k];
-            }
+            keys_out[dst] = key[k];
+            vals_out[dst] = val[k];
         }
     }
 }
@@ -571,25 +572,24 @@ __global__ void __launch_bounds__(kTreeThreads)
     __shared__ uint2 s_left[kMostLeft];
     __shared__ uint32_t s_nleft;
     wait_for_previous();
-    // the sort gave up: the keys are not ordered.  (One answer for the block: another
-    // block's wait below may give up meanwhile, and what a part of the block left out
-    // the rest would read.)
-    if (__syncthreads_or(halted(err) ? 1 : 0)) return;
     const uint32_t t = threadIdx.x, first = blockIdx.x * kTreeThreads, i = first + t;
     const uint32_t here = min(kTreeThreads, n - first);
+    const bool stop = halted(err);  // the sort gave up: the keys are not ordered
     uint32_t *s_key = tsm, *s_met = tsm + kTreeThreads;
     const Merged merged{reinterpret_cast<uint2*>(tsm + 2 * kTreeThreads),
                         reinterpret_cast<float*>(tsm + 10 * kTreeThreads), kTreeThreads};
     Box b{};
     uint32_t key = 0;
-    if (i < n) {
+    if (i < n && !stop) {
         s_key[t] = key = keys[i];
         b = tree.leaf_box(i);
     }
     s_met[t] = 0;
     merged.range[t] = make_uint2(kNone, 0);
     if (t == 0) s_nleft = 0;
-    __syncthreads();
+    // (One answer for the block: another block's wait below may give up meanwhile, and
+    // what a part of the block left out the rest would read.)
+    if (__syncthreads_or(stop ? 1 : 0)) return;
     if (i < n) {
         const uint32_t after = t + 1 < here ? s_key[t + 1] : i + 1 < n ? keys[i + 1] : 0u;
         s_delta[t + 1] = i + 1 < n ? delta(key, after, i) : -1;
