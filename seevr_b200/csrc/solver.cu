@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(kSolverThreads)
 
 // a contact side's bundle-local body, flags and rank
 // (Free: the body is not written and orders nothing; Skip: both masses infinite;
-// Same, with Free, on side a: side b is the same dynamic body, whose velocities
-// side a reads at every update and which b writes last)
+// Same, with Free, on side a: side b is the same dynamic body, which a reads at every
+// update and b writes)
 constexpr uint32_t kSideBody = 0xFFFu, kSideFree = 1u << 12, kSideSkip = 1u << 13,
                    kSideSame = 1u << 14, kRankShift = 16, kMaxRank = 0xFFFFu;
 static_assert(kWarpMaxBodies <= kSideBody, "body field too narrow");
@@ -396,9 +396,17 @@ struct Chunks {
     uint32_t n, levels;
 };
 template <uint32_t W>
-__device__ __forceinline__ Chunks build_levels(const uint32_t* info, const FlowBodies& B, uint32_t nc,
+__device__ __noinline__ Chunks build_levels(const uint32_t* info, const FlowBodies B, uint32_t nc,
                                                uint32_t chained, uint32_t* placed, uint32_t* order,
                                                Chunks chunks, uint32_t* counts) {
+    // (A call of its own, and the sweep's two kinds of records apart: in one piece with
+    // them the rounds' registers were allotted otherwise, 2% of a frame of 100 scenes.)
+    __builtin_assume(__isShared(counts));
+    __builtin_assume(__isShared(B.v));
+    __builtin_assume(__isShared(B.w));
+    __builtin_assume(__isGlobal(placed));
+    __builtin_assume(__isGlobal(chunks.first));
+    __builtin_assume(__isGlobal(chunks.level));
     const uint32_t t = threadIdx.x;
     for (uint32_t i = t; i < nc; i += 32 * W) {
         const bool lone = degree_of(info, B, i) <= 1u;
@@ -446,10 +454,11 @@ __device__ __forceinline__ Chunks build_levels(const uint32_t* info, const FlowB
 struct Recs {
     float4 *p, *stage;
     uint32_t half, stride, step, slots;
+    bool fits;
     static constexpr uint32_t kPad = 7;  // contacts' worth of padding at most
     // room: float4s of shared memory; most: threads
     __device__ __forceinline__ Recs(float4* shared, uint32_t room, float4* global, uint32_t nc, uint32_t most) {
-        const bool fits = (nc + kPad) * kRecWords <= room;
+        fits = (nc + kPad) * kRecWords <= room;
         p = fits ? shared : global;
         half = (nc + 1) / 2;
         half = fits ? half + (12u - half % 8u) % 8u : kRecWords;  // 4 modulo 8
@@ -487,6 +496,7 @@ __device__ __forceinline__ void flow_sweep(const FlowArgs& f, const FlowBodies& 
     Rec h = load_rec(f.rec.at(c), f.rec.stride);
     uint32_t xa = f.info[2 * c], xb = f.info[2 * c + 1];
     uint32_t da = 0, db = 0, ka = 0, kb = 0;  // degrees, counts to wait for
+    bool ra = false, rb = false;              // sides read in every round
     State x{};
     bool live = i < f.nc && f.iters > 0 && !(xa & kSideSkip);
     auto degree = [&](uint32_t y) { return y & kSideFree ? 0u : *B.count(y & kSideBody); };
@@ -497,15 +507,19 @@ __device__ __forceinline__ void flow_sweep(const FlowArgs& f, const FlowBodies& 
             da = d & 0xFFFFu;
             db = d >> 16;
         }
-        ka = da * (it + 1) + (xa >> kRankShift);
+        const bool same = (xa & kSideSame) != 0u;  // side a is side b's body, its turns b's
+        if (same) da = db;
+        ka = da * (it + 1) + ((same ? xb : xa) >> kRankShift);
         kb = db * (it + 1) + (xb >> kRankShift);
-        // (the others are read in every round, and so is a body that is both sides)
-        if ((!kSeveral || (xa & kSideFree)) && !(xa & kSideSame)) {
+        // a body that no other contact moves keeps its velocities in registers
+        ra = same || ((kSeveral || da > 1u) && !(xa & kSideFree));
+        rb = (kSeveral || db > 1u) && !(xb & kSideFree);
+        if (!kSeveral || !ra) {
             const float4 v = ld4(B.v + (xa & kSideBody)), o = ld4(B.w + (xa & kSideBody));
             x.va = mk(v.x, v.y, v.z);
             x.wa = mk(o.x, o.y, o.z);
         }
-        if (!kSeveral || (xb & kSideFree)) {
+        if (!kSeveral || !rb) {
             const float4 v = ld4(B.v + (xb & kSideBody)), o = ld4(B.w + (xb & kSideBody));
             x.vb = mk(v.x, v.y, v.z);
             x.wb = mk(o.x, o.y, o.z);
@@ -529,24 +543,19 @@ __device__ __forceinline__ void flow_sweep(const FlowArgs& f, const FlowBodies& 
     // the first unfinished update of the sequence is ready in every round, so
     // iters * nc rounds are enough
     for (uint64_t round = 0, cap = uint64_t(f.iters) * f.nc; round <= cap; ++round) {
-        // a body that no other contact moves keeps its velocities in registers
         bool ready = live;
         const uint32_t la = xa & kSideBody, lb = xb & kSideBody;
-        if (live && (kSeveral || da > 1u) && !(xa & kSideFree)) {
+        if (live && ra) {
             const float4 v = ld4(B.v + la), o = ld4(B.w + la);
             ready = __float_as_uint(v.w) == ka;
             x.va = mk(v.x, v.y, v.z);
             x.wa = mk(o.x, o.y, o.z);
         }
-        if (live && (kSeveral || db > 1u) && !(xb & kSideFree)) {
+        if (live && rb) {
             const float4 v = ld4(B.v + lb), o = ld4(B.w + lb);
             ready = ready && __float_as_uint(v.w) == kb;
             x.vb = mk(v.x, v.y, v.z);
             x.wb = mk(o.x, o.y, o.z);
-        }
-        if (xa & kSideSame) {
-            x.va = x.vb;
-            x.wa = x.wb;
         }
         const uint32_t left = *f.left;
         part_sync<W>(f.threads);  // every read of the round before its writes
@@ -606,6 +615,15 @@ template <uint32_t W>
 __device__ __forceinline__ void level_sweep(const FlowArgs& f, const FlowBodies& B, const Chunks& chunks) {
     const uint32_t lane = threadIdx.x & 31u;
     const bool staged = threadIdx.x < f.rec.slots;
+    auto record = [&](uint32_t c) {
+        const float4* p = f.rec.at(c);
+        if (f.rec.fits) {
+            __builtin_assume(__isShared(p));
+            return load_rec(p, f.rec.stride);
+        }
+        __builtin_assume(__isGlobal(p));
+        return load_rec(p);
+    };
     float4* const slot = f.rec.stage + threadIdx.x;
     // a chunk of this warp's: its turn (kNone: none), this lane's contact and its sides
     struct Part {
@@ -649,7 +667,7 @@ __device__ __forceinline__ void level_sweep(const FlowArgs& f, const FlowBodies&
     read_sides(cur);
     read_sides(next);
     Rec h{};
-    if (cur.c != kNone) h = load_rec(f.rec.at(cur.c), f.rec.stride);
+    if (cur.c != kNone) h = record(cur.c);
     auto advance = [&] {  // cur <- next
         cur = next;
         next = read_part();
@@ -684,12 +702,12 @@ __device__ __forceinline__ void level_sweep(const FlowArgs& f, const FlowBodies&
             advance();
             copies_done();
             if (cur.c != kNone)
-                h = staged ? load_rec(slot, f.rec.slots) : load_rec(f.rec.at(cur.c), f.rec.stride);
+                h = staged ? load_rec(slot, f.rec.slots) : record(cur.c);
         }
         part_sync<W>(32 * W);
         if (later) {
             advance();
-            if (cur.c != kNone) h = load_rec(f.rec.at(cur.c), f.rec.stride);
+            if (cur.c != kNone) h = record(cur.c);
         }
     }
 }
@@ -747,9 +765,10 @@ struct RunShared {
 // The solve of a run of nc contacts by a block of W warps, the bodies' velocities and
 // the sides' words in place, left and ticket zero.  c0: the run's place in the scratch
 // lists; contact(i), body(l): the contact and body that i and l stand for; lam: the
-// impulses, zero before; deg: nc words.  Mode COLORED where a body needs more than 32 colours: contact
-// order, or (fall_back false) nothing is done and the result is false.
-template <uint32_t W, class Contact, class Body>
+// impulses, zero before; deg: nc words.  Mode COLORED where a body needs more than 32
+// colours: contact order, or (fall_back false) nothing is done and the result is false.
+// kLevels: there may be more than kSweepFrom contacts per lane in contact order.
+template <uint32_t W, bool kLevels, class Contact, class Body>
 __device__ __forceinline__ bool solve_run(const World& w, const Consts& k, const Scratch& s,
                                           uint32_t mode, float dt, uint32_t c0, uint32_t nc,
                                           uint32_t nbs, const FlowBodies& B, uint32_t* info,
@@ -780,7 +799,7 @@ __device__ __forceinline__ bool solve_run(const World& w, const Consts& k, const
                 if (lane < nc) order[lane] = lane;
             } else {
                 chained = count_chained(info, B, nc);
-                by_level = W > 1 && ok && !coloured && chained > kSweepFrom * kThreads;
+                by_level = kLevels && ok && !coloured && chained > kSweepFrom * kThreads;
                 if (!by_level)
                     order_contacts(info, B, nc, chained, kThreads, coloured ? s.s_order + c0 : nullptr, order);
             }
@@ -804,7 +823,7 @@ __device__ __forceinline__ bool solve_run(const World& w, const Consts& k, const
     __syncthreads();
     if (sh.failed && !fall_back) return false;
     Chunks chunks{s.s_order + c0, s.s_lvl_start + c0, 0u, 0u};
-    if (W > 1 && sh.by_level) {
+    if (kLevels && sh.by_level) {
         chunks = build_levels<W>(info, B, nc, sh.chained, deg, order, chunks, sh.placed);
         __syncthreads();
     }
@@ -839,7 +858,7 @@ __device__ __forceinline__ bool solve_run(const World& w, const Consts& k, const
         const FlowArgs f{chained, role * 32 + lane, kThreads, 32u * min(W, (chained + 31) / 32),
                          k.pgs_iterations, order, info, rec, lam, deg, &sh.left};
         if (role * 32 < chained) {  // dataflow rounds, by the warps that own chained contacts
-            if (W > 1 && sh.by_level)
+            if (kLevels && sh.by_level)
                 level_sweep<W>(f, B, chunks);
             else if (chained > kThreads)
                 flow_sweep<W, true>(f, B);
@@ -904,7 +923,7 @@ __global__ void __launch_bounds__(32 * W, 12 / W)
     }
     if (t == 0) sh.left = sh.ticket = 0;
     __syncthreads();
-    solve_run<W>(
+    solve_run<W, (W > 1)>(
         w, k, s, mode, dt, c0, nc, nbs, B, info, order, rec, w.lambda + c0, s.s_abp + c0, bundle,
         true, sh,
         [&](uint32_t i) { return c0 + i; }, [&](uint32_t l) { return b0 + l; });
@@ -1016,7 +1035,7 @@ __global__ void __launch_bounds__(32 * kIslandWarps, 12 / kIslandWarps)
             }
             __syncthreads();
             const uint32_t slots = sh_slots;
-            const bool done = solve_run<kIslandWarps>(
+            const bool done = solve_run<kIslandWarps, false>(
                 w, k, s, mode, dt, p0, nc, slots, B, info, order, rec, lam, deg, sh_window, false,
                 sh, [&](uint32_t i) { return perm[p0 + i]; },
                 [&](uint32_t l) { return list[l] & 0x7FFFFFFFu; });
@@ -1052,7 +1071,8 @@ int launch_island_flow(const World& w, const Consts& k, const Scratch& s, uint32
 }
 
 constexpr uint32_t kSolverMaxSmem = 160 * 1024;
-constexpr uint32_t kFlowMaxSmem = 120 * 1024, kFlowSmem = 192 * 1024;
+constexpr uint32_t kFlowMaxSmem = 120 * 1024, kFlowSmem = 192 * 1024,
+                   kFlowSmemGroups = 150 * 1024;
 
 cudaError_t init_solver() {
     for (const void* f : {reinterpret_cast<const void*>(k_solver_flow<1>),
@@ -1087,13 +1107,16 @@ cudaError_t init_solver() {
 // KB.  With 228 KB two blocks of four warps fitted (77,824 bytes each, 454 us for 4,096
 // scenes in 512-body bundles; 377 with three), and three of 76,700 bytes leave the SM's
 // other kernels next to no L1: with eight groups 13.4 ms per frame, 11.2 with 192 KB.
+// Scene groups' bundles of up to 512 bodies, whose records mostly fit, share 150 KB: 8
+// groups of 128 scenes 4.29 ms per frame with 192 KB, 4.26 with 150.
 static void launch_flow(const World& w, const Consts& k, const Scratch& s, uint32_t mode, float dt,
                         uint32_t nbmax, cudaStream_t st) {
     const uint32_t warps = nbmax <= 128                                            ? 1u
                            : nbmax <= 256                                          ? 2u
                            : nbmax <= 512 || w.nbundles > 148u || s.order_pairs != 0 ? 4u
                                                                                    : 8u;
-    const uint32_t part = warps <= 4 ? kFlowSmem / (12 / warps) - 1024u - 128u : kFlowMaxSmem;
+    const uint32_t share = s.order_pairs != 0 && nbmax <= 512 ? kFlowSmemGroups : kFlowSmem;
+    const uint32_t part = warps <= 4 ? share / (12 / warps) - 1024u - 128u : kFlowMaxSmem;
     const uint32_t smem = std::max(part, 32 * nbmax) & ~15u;
     switch (warps) {
         case 1: launch_after(k_solver_flow<1>, w.nbundles, 32, smem, st, w, k, s, mode, dt, smem / 16); break;
