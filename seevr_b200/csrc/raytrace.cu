@@ -373,6 +373,11 @@ __device__ __forceinline__ float schlick(float cos_theta, float r0) {  // 157-15
 }
 
 constexpr uint32_t kRtThreads = 128;
+// Triangles from which wide nodes are built and traversed: below, a lane's ray is so
+// short that waiting for others costs more than it saves.  Frames of 640x480 with the
+// binary / the wide tree: 24 triangles 444 / 569 us, 1,060 613 / 680, 1,584 699 / 675,
+// 15,732 1,656 / 1,262.
+constexpr uint32_t kWideFrom = 1500;
 // Lanes of a warp whose ray is done at which their hits are shaded, and lanes at inner
 // nodes up to which a warp goes on to the leaves.  A frame is bound by issue (68% of
 // the slots) with few lanes active per instruction (6 of 32 before), so both are
@@ -397,6 +402,8 @@ __device__ __forceinline__ void camera_ray(const RtArgs& g, uint32_t px, uint32_
 // Sample paths (raytrace.comp:192-270).  Item q
 // is sample q % 16 of pixel q / 16 (row-major), so a warp's first paths are
 // two neighbouring pixels' samples; its colour goes to samples[3q..3q+2].
+// Without kWide: a lane traces the binary tree, one bounce per step of the warp.
+template <bool kWide>
 __global__ void __launch_bounds__(kRtThreads) k_rt_paths(RtArgs g, const NodeP* __restrict__ nodes,
                                                          const Wide* __restrict__ wide,
                                                          const TriP* __restrict__ tris,
@@ -406,14 +413,14 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_paths(RtArgs g, const NodeP* 
                                                          uint32_t nitems) {
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned full = 0xFFFFFFFFu;
-    const bool plain = *bad != 0u;  // only the shader's own traversal
+    const bool plain = kWide && *bad != 0u;  // only the shader's own traversal
     enum : uint32_t { kIdle, kTracing, kWaiting };
     uint32_t mode = kIdle;
     bool drained = false;
     uint32_t item = 0, seed = 0, bounce = 0;
     f3 ro = mk(0.f, 0.f, 0.f), rd = ro, inv = ro, throughput = ro, color = ro;
     Hit h{};
-    uint2 stack[kWideStack];  // node or leaf, bits of its entry
+    uint2 stack[kWide ? kWideStack : 1];  // node or leaf, bits of its entry
     int sp = 0;
     uint32_t cur = kNone;  // the node or leaf the lane is at
     // Pushes the children of the inner node cur that the ray enters, last to first, so
@@ -436,6 +443,10 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_paths(RtArgs g, const NodeP* 
     };
     // Starts the ray (ro, rd).
     auto launch = [&] {
+        if constexpr (!kWide) {
+            mode = kTracing;
+            return;
+        }
         h.t = 1e10f;
         h.normal = mk(0.f, 1.f, 0.f);
         h.tri = 0xFFFFFFFFu;
@@ -478,40 +489,47 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_paths(RtArgs g, const NodeP* 
         // ---- steps of the rays, until enough of them are done ----
         const int busy = __popc(__ballot_sync(full, mode != kIdle));
         if (busy == 0) break;
-        // the nearest entry left on the stack that is still nearer than the hit
-        auto pop = [&] {
-            cur = kNone;
-            while (sp > 0) {
-                const uint2 e = stack[--sp];
-                if (__uint_as_float(e.y) < h.t) {
-                    cur = e.x;
-                    break;
-                }
-            }
-            if (cur == kNone) mode = kWaiting;
-        };
-        while (true) {
-            const int tracing = __popc(__ballot_sync(full, mode == kTracing));
-            if (tracing == 0 || busy - tracing >= kShadeLanes) break;
-            // inner nodes, until few lanes are at one
-            while (true) {
-                const bool inner = mode == kTracing && cur < kMulti;
-                if (__popc(__ballot_sync(full, inner)) <= kInnerLanes) break;
-                if (!inner) continue;
-                visit();
-                pop();
-            }
+        if constexpr (!kWide) {
             if (mode == kTracing) {
-                if (cur & kLeafBit) {
-                    hit_triangle(tris, cur & ~kLeafBit, ro, rd, h);
-                } else if (cur & kMulti) {
-                    const NodeP n = nodes[cur & kNodeMask];
-                    const uint32_t lf = __float_as_uint(n.lo.w), cnt = __float_as_uint(n.hi.w) & ~kLeafBit;
-                    for (uint32_t i = 0; i < cnt; ++i) hit_triangle(tris, lf + i, ro, rd, h);
-                } else {
-                    visit();
+                trace(nodes, tris, ro, rd, h.t, h.normal, h.tri, h.front);
+                mode = kWaiting;
+            }
+        } else {
+            // the nearest entry left on the stack that is still nearer than the hit
+            auto pop = [&] {
+                cur = kNone;
+                while (sp > 0) {
+                    const uint2 e = stack[--sp];
+                    if (__uint_as_float(e.y) < h.t) {
+                        cur = e.x;
+                        break;
+                    }
                 }
-                pop();
+                if (cur == kNone) mode = kWaiting;
+            };
+            while (true) {
+                const int tracing = __popc(__ballot_sync(full, mode == kTracing));
+                if (tracing == 0 || busy - tracing >= kShadeLanes) break;
+                // inner nodes, until few lanes are at one
+                while (true) {
+                    const bool inner = mode == kTracing && cur < kMulti;
+                    if (__popc(__ballot_sync(full, inner)) <= kInnerLanes) break;
+                    if (!inner) continue;
+                    visit();
+                    pop();
+                }
+                if (mode == kTracing) {
+                    if (cur & kLeafBit) {
+                        hit_triangle(tris, cur & ~kLeafBit, ro, rd, h);
+                    } else if (cur & kMulti) {
+                        const NodeP n = nodes[cur & kNodeMask];
+                        const uint32_t lf = __float_as_uint(n.lo.w), cnt = __float_as_uint(n.hi.w) & ~kLeafBit;
+                        for (uint32_t i = 0; i < cnt; ++i) hit_triangle(tris, lf + i, ro, rd, h);
+                    } else {
+                        visit();
+                    }
+                    pop();
+                }
             }
         }
         if (mode != kWaiting) continue;
@@ -692,10 +710,12 @@ seevr_status seevr_raytrace(const seevr_rt_bindings* b, const seevr_rt_params* p
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rt_paths, kRtThreads, 0);
+    const bool few = p->num_triangles < kWideFrom;  // the binary tree only
+    const auto paths = few ? k_rt_paths<false> : k_rt_paths<true>;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, paths, kRtThreads, 0);
     // work arrays, stream-ordered: wide and binary nodes, triangles, per-sample
     // colours, parents, the path ticket
-    const size_t wide_bytes = size_t(nnodes) * sizeof(Wide), node_bytes = size_t(nnodes) * sizeof(NodeP),
+    const size_t wide_bytes = few ? 0 : size_t(nnodes) * sizeof(Wide), node_bytes = size_t(nnodes) * sizeof(NodeP),
                  tri_bytes = size_t(p->num_triangles) * sizeof(TriP);
     const size_t sample_bytes = (size_t(nitems) * 3 * sizeof(float) + 15) & ~size_t(15);
     const size_t parent_bytes = size_t(nnodes) * sizeof(uint32_t);
@@ -719,18 +739,18 @@ seevr_status seevr_raytrace(const seevr_rt_bindings* b, const seevr_rt_params* p
     uint32_t* bad = ticket + 1;
     const uint32_t cap = uint32_t(std::max(sms, 1)) * 8u;
     const uint32_t nblocks = std::min((nnodes + 255) / 256, cap);
-    cudaMemsetAsync(parent, 0xFF, parent_bytes, st);
-    // a tree of one leaf has no inner node
-    cudaMemsetAsync(ticket, 0, sizeof(uint32_t), st);
-    cudaMemsetAsync(bad, nnodes == 1 ? 1 : 0, sizeof(uint32_t), st);
+    cudaMemsetAsync(ticket, 0, 2 * sizeof(uint32_t), st);
     k_rt_pack_nodes<<<nblocks, 256, 0, st>>>(g, nnodes, nodes);
     k_rt_pack_tris<<<std::min((p->num_triangles + 255) / 256, cap), 256, 0, st>>>(g, tris);
-    k_rt_parents<<<nblocks, 256, 0, st>>>(g, nnodes, parent, bad);
-    k_rt_check<<<nblocks, 256, 0, st>>>(g, nodes, nnodes, parent, bad);
-    k_rt_wide<<<nblocks, 256, 0, st>>>(g, nodes, nnodes, bad, wide);
+    if (!few) {
+        cudaMemsetAsync(parent, 0xFF, parent_bytes, st);
+        k_rt_parents<<<nblocks, 256, 0, st>>>(g, nnodes, parent, bad);
+        k_rt_check<<<nblocks, 256, 0, st>>>(g, nodes, nnodes, parent, bad);
+        k_rt_wide<<<nblocks, 256, 0, st>>>(g, nodes, nnodes, bad, wide);
+    }
     const uint32_t resident = uint32_t(std::max(sms, 1)) * uint32_t(std::max(per_sm, 1));
     const uint32_t blocks = std::min((nitems + kRtThreads - 1) / kRtThreads, resident);
-    k_rt_paths<<<blocks, kRtThreads, 0, st>>>(g, nodes, wide, tris, samples, ticket, bad, nitems);
+    paths<<<blocks, kRtThreads, 0, st>>>(g, nodes, wide, tris, samples, ticket, bad, nitems);
     k_rt_resolve<<<std::min(uint32_t((npix + 255) / 256), cap), 256, 0, st>>>(g, samples);
     e = cudaGetLastError();
     cudaFreeAsync(work, st);
