@@ -34,7 +34,7 @@ namespace {
 
 constexpr uint32_t kIslandThreads = 128;
 // Sort passes (8 bits each) for roots below nb and, above them, the key of skipped
-// contacts: 2 for 65,535 bodies.
+// contacts: 1 below 255 bodies, 2 below 65,535.
 inline uint32_t key_passes(uint32_t nb) {
     uint32_t p = 1;
     while (p < 4 && nb >= (1u << (8 * p)) - 1u) ++p;

@@ -381,7 +381,7 @@ constexpr uint32_t kWideFrom = 1500;
 // Lanes of a warp whose ray is done at which their hits are shaded, and lanes at inner
 // nodes up to which a warp goes on to the leaves.  A frame is bound by issue (68% of
 // the slots) with few lanes active per instruction (6 of 32 before), so both are
-// chosen for full warps: 640x480 over 134,156 triangles 6.28 ms (9.86 ms with the
+// chosen for full warps: 640x480 over 134,156 triangles 6.0 ms (9.5 ms with the
 // binary tree one bounce per step); 7.0 ms with 6 and 4, 7.9 ms with 20 and 0.
 constexpr int kShadeLanes = 20;
 constexpr int kInnerLanes = 10;
