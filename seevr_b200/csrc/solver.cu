@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(kSolverThreads)
 
 // a contact side's bundle-local body, flags and rank
 // (Free: the body is not written and orders nothing; Skip: both masses infinite;
-// Same, with Free, on side a: side b is the same dynamic body, which a reads at every
-// update and b writes)
+// Same, with Free, on side a: side b is the same dynamic body, whose velocities side a
+// takes at every update and which b writes last)
 constexpr uint32_t kSideBody = 0xFFFu, kSideFree = 1u << 12, kSideSkip = 1u << 13,
                    kSideSame = 1u << 14, kRankShift = 16, kMaxRank = 0xFFFFu;
 static_assert(kWarpMaxBodies <= kSideBody, "body field too narrow");
@@ -496,7 +496,6 @@ __device__ __forceinline__ void flow_sweep(const FlowArgs& f, const FlowBodies& 
     Rec h = load_rec(f.rec.at(c), f.rec.stride);
     uint32_t xa = f.info[2 * c], xb = f.info[2 * c + 1];
     uint32_t da = 0, db = 0, ka = 0, kb = 0;  // degrees, counts to wait for
-    bool ra = false, rb = false;              // sides read in every round
     State x{};
     bool live = i < f.nc && f.iters > 0 && !(xa & kSideSkip);
     auto degree = [&](uint32_t y) { return y & kSideFree ? 0u : *B.count(y & kSideBody); };
@@ -507,19 +506,15 @@ __device__ __forceinline__ void flow_sweep(const FlowArgs& f, const FlowBodies& 
             da = d & 0xFFFFu;
             db = d >> 16;
         }
-        const bool same = (xa & kSideSame) != 0u;  // side a is side b's body, its turns b's
-        if (same) da = db;
-        ka = da * (it + 1) + ((same ? xb : xa) >> kRankShift);
+        ka = da * (it + 1) + (xa >> kRankShift);
         kb = db * (it + 1) + (xb >> kRankShift);
-        // a body that no other contact moves keeps its velocities in registers
-        ra = same || ((kSeveral || da > 1u) && !(xa & kSideFree));
-        rb = (kSeveral || db > 1u) && !(xb & kSideFree);
-        if (!kSeveral || !ra) {
+        // (the others are read in every round, and so is a body that is both sides)
+        if ((!kSeveral || (xa & kSideFree)) && !(xa & kSideSame)) {
             const float4 v = ld4(B.v + (xa & kSideBody)), o = ld4(B.w + (xa & kSideBody));
             x.va = mk(v.x, v.y, v.z);
             x.wa = mk(o.x, o.y, o.z);
         }
-        if (!kSeveral || !rb) {
+        if (!kSeveral || (xb & kSideFree)) {
             const float4 v = ld4(B.v + (xb & kSideBody)), o = ld4(B.w + (xb & kSideBody));
             x.vb = mk(v.x, v.y, v.z);
             x.wb = mk(o.x, o.y, o.z);
@@ -543,19 +538,24 @@ __device__ __forceinline__ void flow_sweep(const FlowArgs& f, const FlowBodies& 
     // the first unfinished update of the sequence is ready in every round, so
     // iters * nc rounds are enough
     for (uint64_t round = 0, cap = uint64_t(f.iters) * f.nc; round <= cap; ++round) {
+        // a body that no other contact moves keeps its velocities in registers
         bool ready = live;
         const uint32_t la = xa & kSideBody, lb = xb & kSideBody;
-        if (live && ra) {
+        if (live && (kSeveral || da > 1u) && !(xa & kSideFree)) {
             const float4 v = ld4(B.v + la), o = ld4(B.w + la);
             ready = __float_as_uint(v.w) == ka;
             x.va = mk(v.x, v.y, v.z);
             x.wa = mk(o.x, o.y, o.z);
         }
-        if (live && rb) {
+        if (live && (kSeveral || db > 1u) && !(xb & kSideFree)) {
             const float4 v = ld4(B.v + lb), o = ld4(B.w + lb);
             ready = ready && __float_as_uint(v.w) == kb;
             x.vb = mk(v.x, v.y, v.z);
             x.wb = mk(o.x, o.y, o.z);
+        }
+        if (xa & kSideSame) {
+            x.va = x.vb;
+            x.wa = x.wb;
         }
         const uint32_t left = *f.left;
         part_sync<W>(f.threads);  // every read of the round before its writes
@@ -1072,7 +1072,8 @@ int launch_island_flow(const World& w, const Consts& k, const Scratch& s, uint32
 
 constexpr uint32_t kSolverMaxSmem = 160 * 1024;
 constexpr uint32_t kFlowMaxSmem = 120 * 1024, kFlowSmem = 192 * 1024,
-                   kFlowSmemGroups = 150 * 1024;
+                   kFlowSmemGroups = 150 * 1024, kFlowSmemTwo = 79 * 1024 - 128,
+                   kTwoPerSm = 2 * 148 + 148 / 5;
 
 cudaError_t init_solver() {
     for (const void* f : {reinterpret_cast<const void*>(k_solver_flow<1>),
@@ -1108,7 +1109,11 @@ cudaError_t init_solver() {
 // scenes in 512-body bundles; 377 with three), and three of 76,700 bytes leave the SM's
 // other kernels next to no L1: with eight groups 13.4 ms per frame, 11.2 with 192 KB.
 // Scene groups' bundles of up to 512 bodies, whose records mostly fit, share 150 KB: 8
-// groups of 128 scenes 4.29 ms per frame with 192 KB, 4.26 with 150.
+// groups of 128 scenes 4.29 ms per frame with 192 KB, 4.26 with 150.  Two blocks of four
+// warps to an SM while that leaves few bundles over, which start as the first ones end: a
+// third block beside the longest chain costs more, and more records fit (1,024 scenes, 306
+// bundles: 4.30 ms per frame with two, 4.14 to 4.51 with three, by where the chain lies;
+// 1,150 scenes 4.52 and 4.38).
 static void launch_flow(const World& w, const Consts& k, const Scratch& s, uint32_t mode, float dt,
                         uint32_t nbmax, cudaStream_t st) {
     const uint32_t warps = nbmax <= 128                                            ? 1u
@@ -1116,7 +1121,8 @@ static void launch_flow(const World& w, const Consts& k, const Scratch& s, uint3
                            : nbmax <= 512 || w.nbundles > 148u || s.order_pairs != 0 ? 4u
                                                                                    : 8u;
     const uint32_t share = s.order_pairs != 0 && nbmax <= 512 ? kFlowSmemGroups : kFlowSmem;
-    const uint32_t part = warps <= 4 ? share / (12 / warps) - 1024u - 128u : kFlowMaxSmem;
+    uint32_t part = warps <= 4 ? share / (12 / warps) - 1024u - 128u : kFlowMaxSmem;
+    if (warps == 4 && s.order_pairs == 0 && w.nbundles <= kTwoPerSm) part = kFlowSmemTwo;
     const uint32_t smem = std::max(part, 32 * nbmax) & ~15u;
     switch (warps) {
         case 1: launch_after(k_solver_flow<1>, w.nbundles, 32, smem, st, w, k, s, mode, dt, smem / 16); break;
